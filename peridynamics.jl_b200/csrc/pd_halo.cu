@@ -176,6 +176,10 @@ extern "C" pd_status pd_halo_unpack(pd_handle* h, int32_t kind, const int32_t* d
     launch_split_u_rows(h->d, d_rows, n_rows, h->stream);
     h->launches++;
   }
+  if (kind == 1 && h->d.cst64) {
+    launch_c_state_rows(h->d, d_rows, n_rows, h->stream);
+    h->launches++;
+  }
   if (kind == 1 && h->material == PD_MAT_CMAT && !h->d.sym) {
     k_halo_kill_bonds<<<halo_blocks(n_rows), 256, 0, h->stream>>>(h->d, d_rows, n_rows);
     h->launches++;

@@ -62,6 +62,12 @@ struct IntDev {
 // force evaluation; phase 0 = all kernels, 1 = the first (BB: the only) kernel, 2 = the
 // second kernel of the state-based materials. Returns the number of kernels launched.
 int launch_force64(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s);
+// the kernels off the serial order (pd_force64_fast.cu): phase 1 (BB: the force), phase 2 where
+// fast64_supported
+bool fast64_supported(const DevBody& d);
+void launch_force64_fast(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s);
+// the phase-B state of rows[0 .. n) (halo rows that received F and P K^-1)
+void launch_c_state_rows(const DevBody& d, const int* rows, long long n, cudaStream_t s);
 int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s);
 bool tma_supported(const DevBody& d);
 int launch_force32_tma(const DevBody& d, int pipe, int kstep, int phase, cudaStream_t s);
