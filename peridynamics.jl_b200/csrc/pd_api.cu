@@ -331,9 +331,44 @@ static pd_status relayout(pd_handle* h, int G) {
   dfree(h, (void*)a.soff); dfree(h, (void*)a.nbr); dfree(h, (void*)a.rev);
   dfree(h, (void*)a.len64); dfree(h, (void*)a.geo); dfree(h, a.bits);
   dfree(h, (void*)a.sc64); dfree(h, (void*)a.sc32);
+  dfree(h, (void*)a.cls); dfree(h, (void*)a.cls_geo); dfree(h, (void*)a.cls_dj);
+  b.cls = nullptr;
+  b.cls_geo = nullptr;
+  b.cls_dj = nullptr;
+  b.ncls = 0;
+  h->cls_tried = false;
   h->d = b;
   h->nslots = nslots;
   destroy_graph(h);
+  return PD_OK;
+}
+
+// The packed FP32 kernels (pipe 5) read the bonds of a body on a regular lattice as one byte each.
+// Looked for once per layout, when the variant is chosen (two passes over the bonds); a body
+// without classes, or without the memory for them, keeps the full bond stream.
+static pd_status ensure_classes(pd_handle* h) {
+  if (h->cls_tried || h->precision == PD_PREC_FP64 || h->cfg.pipe != 5 || !packed_supported(h->d, 1))
+    return PD_OK;
+  h->cls_tried = true;
+  unsigned* cls = nullptr;
+  float4* geo = nullptr;
+  int* dj = nullptr;
+  int ncls = 0;
+  const cudaError_t e = build_classes(h->d, h->nslots, &cls, &geo, &dj, &ncls, h->stream);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return PD_OK;
+  }
+  PD_CUDA(e);
+  if (ncls == 0) return PD_OK;
+  h->allocs.push_back(cls);
+  h->allocs.push_back(geo);
+  h->allocs.push_back(dj);
+  h->d.cls = cls;
+  h->d.cls_geo = geo;
+  h->d.cls_dj = dj;
+  h->d.ncls = ncls;
+  h->version++;
   return PD_OK;
 }
 
@@ -1386,6 +1421,7 @@ extern "C" pd_status pd_autotune(pd_handle* h, int32_t* group_out, int32_t* bloc
   std::vector<Cand> cands;
   // five evaluations of the current configuration after one warm-up
   auto time_cfg = [&](float* out) -> pd_status {
+    PD_TRY(ensure_classes(h));
     launch_force(h, 0, 0);
     cudaEventRecord(e0, h->stream);
     for (int r = 0; r < 5; r++) launch_force(h, 0, 0);
@@ -1443,6 +1479,7 @@ extern "C" pd_status pd_autotune(pd_handle* h, int32_t* group_out, int32_t* bloc
     if (c.ms < best) { best = c.ms; bestc = c.c; }
   PD_TRY(relayout(h, bestc.group));
   h->cfg = bestc;
+  PD_TRY(ensure_classes(h));
   destroy_graph(h);
   if (group_out) *group_out = bestc.group;
   if (block_out) *block_out = bestc.block;
@@ -1566,9 +1603,10 @@ extern "C" pd_status pd_set_pipeline(pd_handle* h, int32_t pipe) {
     return fail(PD_ERR_ARG, "the packed-pair kernels are FP32 ones");
   if (pipe >= 1 && pipe <= 3 && (h->precision != PD_PREC_FP32_KAHAN || !tma_supported(h->d)))
     return fail(PD_ERR_ARG, "the staged bond stream needs the FP32 path, one lane per point and BB or OSB");
+  PD_CUDA(cudaSetDevice(h->device));
   h->cfg.pipe = pipe;
   destroy_graph(h);
-  return PD_OK;
+  return ensure_classes(h);
 }
 
 // helpers shared with pd_nk.cu

@@ -90,6 +90,11 @@ struct DevBody {
   const int* rev;    // revk
   const double* len64;
   const float4* geo;
+  // bond classes (pd_classes.cu): one byte a bond into tables of ncls entries; ncls = 0: none
+  const unsigned* cls;
+  const float4* cls_geo;
+  const int* cls_dj;
+  int ncls;
   const double4* X0;
   double4* cur;
   unsigned int* meta;

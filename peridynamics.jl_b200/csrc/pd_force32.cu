@@ -20,6 +20,7 @@
 #include "pd_common.cuh"
 #include "pd_launch.h"
 #include "pd_pack.cuh"
+#include "pd_stream32.cuh"
 
 namespace pd {
 
@@ -946,10 +947,11 @@ __device__ __forceinline__ void bond_c(const float4& g, const float4& hj, const 
   B.eps = __fdividef(fmaf(2.f, xd, dd), l + B.L) * B.rL;
 }
 
-template <bool FULLK, bool LIN>
+template <bool CLS, bool FULLK, bool LIN>
 __global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kstep) {
   using namespace pack;
-  if (d.ctrl->err) return;
+  __shared__ ClassTable tab;
+  if (!stream_begin<CLS>(d, &tab)) return;
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -967,9 +969,6 @@ __global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kste
     const float nhz = -hi.z, nlz = -lo.z;
     const float epsc = P.epscf, id = P.inv_delta, vs = P.vscale;
     const float2 id2 = make_float2(id, id);
-    const int* pn = d.nbr + sbase + lane;
-    const float4* pg = d.geo + sbase + lane;
-    unsigned* pw = d.bits + (sbase >> 5);
     KSum2 K01, K23, K45;        // FULLK: (xx, yy), (zz, xy), (xz, yz)
     // rows x, y of column c of the displacement-gradient sum, and row z: plain FP32 sums (with
     // compensated sums phase A took 0.648 against 0.594 ms on the 1M-point CMat block, and the
@@ -979,28 +978,17 @@ __global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kste
     float Hz[3] = {0.f, 0.f, 0.f};
     float dK[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     int na = 0;
-    int nj0 = self, nj1 = self;
-    float4 ng0 = make_float4(0.f, 0.f, 0.f, 1.f), ng1 = ng0;
-    unsigned nw0 = 0u, nw1 = 0u;
-    auto load_pair = [&](int r) {
-      const bool two = r + 1 < rows;
-      nw0 = pw[r];
-      nw1 = two ? pw[r + 1] : 0u;
-      nj0 = ld_stream(pn + 32 * r);
-      ng0 = ld_stream(pg + 32 * r);
-      if (two) { nj1 = ld_stream(pn + 32 * r + 32); ng1 = ld_stream(pg + 32 * r + 32); }
-      else { nj1 = self; ng1 = make_float4(0.f, 0.f, 0.f, 1.f); }
-    };
-    if (rows > 0) load_pair(0);
+    Stream32<CLS, true> st(d, &tab, s, sbase, rows, lane, self);
     for (int r = 0; r < rows; r += 2) {
       const bool two = r + 1 < rows;
-      const unsigned w0 = nw0, w1 = nw1;
-      const bool a0 = (w0 >> lane) & 1u, a1 = (w1 >> lane) & 1u;
-      const int j0 = a0 ? nj0 : self, j1 = a1 ? nj1 : self;
-      const float4 g0 = ng0, g1 = ng1;
+      unsigned w0, w1;
+      bool a0, a1;
+      int j0, j1;
+      float4 g0, g1;
+      st.take(r, w0, w1, a0, a1, j0, j1, g0, g1);
       const float4 hj0 = __ldg(d.uhi + j0), lj0 = __ldg(d.ulo + j0);
       const float4 hj1 = __ldg(d.uhi + j1), lj1 = __ldg(d.ulo + j1);
-      if (r + 2 < rows) load_pair(r + 2);
+      if (r + 2 < rows) st.load(r + 2);
       bool act0, act1;
 #pragma unroll
       for (int u = 0; u < 2; u++) {
@@ -1036,8 +1024,8 @@ __global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kste
       const unsigned c0 = __ballot_sync(0xffffffffu, act0);
       const unsigned c1 = __ballot_sync(0xffffffffu, act1);
       if (lane == 0) {
-        if (c0 != w0) pw[r] = c0;
-        if (two && c1 != w1) pw[r + 1] = c1;
+        if (c0 != w0) d.bits[(sbase >> 5) + r] = c0;
+        if (two && c1 != w1) d.bits[(sbase >> 5) + r + 1] = c1;
       }
     }
     bool killed = false;
@@ -1092,10 +1080,11 @@ __global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kste
   }
 }
 
-template <bool LIN>
+template <bool CLS, bool LIN>
 __global__ void __launch_bounds__(256, PD_MINB_CQB) k_c_b32q(DevBody d, int kstep) {
   using namespace pack;
-  if (d.ctrl->err) return;
+  __shared__ ClassTable tab;
+  if (!stream_begin<CLS>(d, &tab)) return;
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -1112,35 +1101,22 @@ __global__ void __launch_bounds__(256, PD_MINB_CQB) k_c_b32q(DevBody d, int kste
     const float nhz = -hi.z, nlz = -lo.z;
     const float4 ci0 = d.cst32[3 * (long long)self], ci1 = d.cst32[3 * (long long)self + 1],
                  ci2 = d.cst32[3 * (long long)self + 2];
-    const int* pn = d.nbr + sbase + lane;
-    const float4* pg = d.geo + sbase + lane;
-    const unsigned* pw = d.bits + (sbase >> 5);
     KSum2 bxy;
     KSum1 bz;
-    int nj0 = self, nj1 = self;
-    float4 ng0 = make_float4(0.f, 0.f, 0.f, 1.f), ng1 = ng0;
-    unsigned nw0 = 0u, nw1 = 0u;
-    auto load_pair = [&](int r) {
-      const bool two = r + 1 < rows;
-      nw0 = ld_stream(pw + r);
-      nw1 = two ? ld_stream(pw + r + 1) : 0u;
-      nj0 = ld_stream(pn + 32 * r);
-      ng0 = ld_stream(pg + 32 * r);
-      if (two) { nj1 = ld_stream(pn + 32 * r + 32); ng1 = ld_stream(pg + 32 * r + 32); }
-      else { nj1 = self; ng1 = make_float4(0.f, 0.f, 0.f, 1.f); }
-    };
-    if (rows > 0) load_pair(0);
+    Stream32<CLS, false> st(d, &tab, s, sbase, rows, lane, self);
     for (int r = 0; r < rows; r += 2) {
-      const bool a0 = (nw0 >> lane) & 1u, a1 = (nw1 >> lane) & 1u;
-      const int j0 = a0 ? nj0 : self, j1 = a1 ? nj1 : self;
-      const float4 g0 = ng0, g1 = ng1;
+      unsigned w0, w1;
+      bool a0, a1;
+      int j0, j1;
+      float4 g0, g1;
+      st.take(r, w0, w1, a0, a1, j0, j1, g0, g1);
       const float4 hj0 = __ldg(d.uhi + j0), lj0 = __ldg(d.ulo + j0);
       const float4 hj1 = __ldg(d.uhi + j1), lj1 = __ldg(d.ulo + j1);
       const float4* cj0 = d.cst32 + 3 * (long long)j0;
       const float4* cj1 = d.cst32 + 3 * (long long)j1;
       const float4 c00 = __ldg(cj0), c01 = __ldg(cj0 + 1), c02 = __ldg(cj0 + 2);
       const float4 c10 = __ldg(cj1), c11 = __ldg(cj1 + 1), c12 = __ldg(cj1 + 2);
-      if (r + 2 < rows) load_pair(r + 2);
+      if (r + 2 < rows) st.load(r + 2);
 #pragma unroll
       for (int u = 0; u < 2; u++) {
         const float4& g = u ? g1 : g0;
@@ -1265,6 +1241,24 @@ static int launch_osb32(const DevBody& d, const LaunchCfg& c, int G, int grid, i
   return launches;
 }
 
+template <bool CLS>
+static void launch_c_a32q(const DevBody& d, const LaunchCfg& c, int grid, int kstep, cudaStream_t s) {
+  const bool lin = d.kernel == KER_LINEAR;
+  if (c.fullk) {
+    if (lin) k_c_a32q<CLS, true, true><<<grid, c.block, 0, s>>>(d, kstep);
+    else k_c_a32q<CLS, true, false><<<grid, c.block, 0, s>>>(d, kstep);
+  } else {
+    if (lin) k_c_a32q<CLS, false, true><<<grid, c.block, 0, s>>>(d, kstep);
+    else k_c_a32q<CLS, false, false><<<grid, c.block, 0, s>>>(d, kstep);
+  }
+}
+
+template <bool CLS>
+static void launch_c_b32q(const DevBody& d, const LaunchCfg& c, int grid, int kstep, cudaStream_t s) {
+  if (d.kernel == KER_LINEAR) k_c_b32q<CLS, true><<<grid, c.block, 0, s>>>(d, kstep);
+  else k_c_b32q<CLS, false><<<grid, c.block, 0, s>>>(d, kstep);
+}
+
 int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s) {
   const int G = d.lg;
   const int grid = grid_for32(d.nslices, c.block);
@@ -1296,15 +1290,9 @@ int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, c
     if (d.sc32) return launch_osb32<true>(d, c, G, grid, kstep, A, B, s);
     return launch_osb32<false>(d, c, G, grid, kstep, A, B, s);
   }
-  const bool lin = d.kernel == KER_LINEAR;
   if (A && c.pipe == 5 && cq_supported(d, 1)) {
-    if (c.fullk) {
-      if (lin) k_c_a32q<true, true><<<grid, c.block, 0, s>>>(d, kstep);
-      else k_c_a32q<true, false><<<grid, c.block, 0, s>>>(d, kstep);
-    } else {
-      if (lin) k_c_a32q<false, true><<<grid, c.block, 0, s>>>(d, kstep);
-      else k_c_a32q<false, false><<<grid, c.block, 0, s>>>(d, kstep);
-    }
+    if (d.ncls > 0) launch_c_a32q<true>(d, c, grid, kstep, s);
+    else launch_c_a32q<false>(d, c, grid, kstep, s);
     launches++;
   } else if (A) {
     if (d.kernel == KER_LINEAR) {
@@ -1319,8 +1307,8 @@ int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, c
   }
   const bool wan = d.zem == ZEM_WAN;
   if (B && c.pipe == 5 && cq_supported(d, 2)) {
-    if (lin) k_c_b32q<true><<<grid, c.block, 0, s>>>(d, kstep);
-    else k_c_b32q<false><<<grid, c.block, 0, s>>>(d, kstep);
+    if (d.ncls > 0) launch_c_b32q<true>(d, c, grid, kstep, s);
+    else launch_c_b32q<false>(d, c, grid, kstep, s);
     launches++;
   } else if (B) {
     if (wan) {

@@ -21,12 +21,17 @@
 // the stream overlaps the gathers and arithmetic of the pair before it. The stream loads are
 // streaming (evict-first) loads, so that the bond records, read once, leave L2 to the
 // neighbours' point records.
+// Bodies on a regular lattice (at most 256 distinct bond records, pd_classes.cu) stream one byte a
+// bond instead of 20 (template flag CLS, the same bits): on the 1M-point blocks OSB phase A 471 ->
+// 383 us, phase B 486 -> 371 us, BB 471 -> 384 us. DRAM throughput falls from 0.75 of the copy rate
+// to 0.06: these kernels are bound by instruction issue (75 % of the slots in phase A).
 // The arithmetic is the FP32 form of pd_force32.cu (deformed bond vector from the stored
 // reference offset, cancellation-free extension, Kahan sums); roundings differ from the
 // two-row kernels only in the order of a few operations.
 #include "pd_common.cuh"
 #include "pd_launch.h"
 #include "pd_pack.cuh"
+#include "pd_stream32.cuh"
 
 namespace pd {
 
@@ -80,13 +85,20 @@ __device__ __forceinline__ float omega_pk(int kernel, float delta, float L, floa
 #ifndef PD_MINB_QB
 #define PD_MINB_QB 3
 #endif
+// phase B on bond classes holds no geometry record between its load and its use: 4 blocks (63
+// registers) take 371 us on the 1M-point block, 3 blocks 426 us, 5 blocks 569 us (spills); phase A
+// and BB stay at 4 (383 us each; 446 and 499 us at 5)
+#ifndef PD_MINB_QBC
+#define PD_MINB_QBC 4
+#endif
 
 // Phase B with the bond stream of the next row pair loaded while the current pair is
 // gathered and computed (one pair of rows ahead): the DRAM latency of the stream overlaps the
 // gathers and arithmetic of the pair before it. MB resident blocks per SM.
-template <bool LIN>
-__global__ void __launch_bounds__(256, PD_MINB_QB) k_osb_b32q(DevBody d, int kstep) {
-  if (d.ctrl->err) return;
+template <bool CLS, bool LIN>
+__global__ void __launch_bounds__(256, CLS ? PD_MINB_QBC : PD_MINB_QB) k_osb_b32q(DevBody d, int kstep) {
+  __shared__ ClassTable tab;
+  if (!stream_begin<CLS>(d, &tab)) return;
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -102,34 +114,20 @@ __global__ void __launch_bounds__(256, PD_MINB_QB) k_osb_b32q(DevBody d, int kst
     const float2 ci = d.cc32[self];
     const float2 nhi = make_float2(-hi.x, -hi.y), nlo = make_float2(-lo.x, -lo.y);
     const float nhz = -hi.z, nlz = -lo.z;
-    const int* pn = d.nbr + sbase + lane;
-    const float4* pg = d.geo + sbase + lane;
-    const unsigned* pw = d.bits + (sbase >> 5);
     KSum2 bxy;
     KSum1 bz;
-    // stream records of the pair (r, r + 1): neighbour (self when inactive), geometry, state
-    int nj0 = self, nj1 = self;
-    float4 ng0 = make_float4(0.f, 0.f, 0.f, 1.f), ng1 = ng0;
-    unsigned nw0 = 0u, nw1 = 0u;
-    auto load_pair = [&](int r) {
-      const bool two = r + 1 < rows;
-      nw0 = ld_stream(pw + r);
-      nw1 = two ? ld_stream(pw + r + 1) : 0u;
-      nj0 = ld_stream(pn + 32 * r);
-      ng0 = ld_stream(pg + 32 * r);
-      if (two) { nj1 = ld_stream(pn + 32 * r + 32); ng1 = ld_stream(pg + 32 * r + 32); }
-      else { nj1 = self; ng1 = make_float4(0.f, 0.f, 0.f, 1.f); }
-    };
-    if (rows > 0) load_pair(0);
+    Stream32<CLS, false> st(d, &tab, s, sbase, rows, lane, self);
     for (int r = 0; r < rows; r += 2) {
-      const bool a0 = (nw0 >> lane) & 1u, a1 = (nw1 >> lane) & 1u;
-      const int j0 = a0 ? nj0 : self, j1 = a1 ? nj1 : self;
-      const float4 g0 = ng0, g1 = ng1;
+      unsigned w0, w1;
+      bool a0, a1;
+      int j0, j1;
+      float4 g0, g1;
+      st.take(r, w0, w1, a0, a1, j0, j1, g0, g1);
       // gathers of this pair, then the stream of the next pair, then the arithmetic
       const float4 hj0 = __ldg(d.uhi + j0), lj0 = __ldg(d.ulo + j0);
       const float4 hj1 = __ldg(d.uhi + j1), lj1 = __ldg(d.ulo + j1);
       const float2 cj0 = __ldg(d.cc32 + j0), cj1 = __ldg(d.cc32 + j1);
-      if (r + 2 < rows) load_pair(r + 2);
+      if (r + 2 < rows) st.load(r + 2);
 #pragma unroll
       for (int u = 0; u < 2; u++) {
         const float4& g = u ? g1 : g0;
@@ -160,9 +158,10 @@ __global__ void __launch_bounds__(256, PD_MINB_QB) k_osb_b32q(DevBody d, int kst
 }
 
 // Phase A with the next row pair's stream loaded one pair ahead (as k_osb_b32q).
-template <bool FULLM, bool LIN>
+template <bool CLS, bool FULLM, bool LIN>
 __global__ void __launch_bounds__(256, PD_MINB_QA) k_osb_a32q(DevBody d, int kstep) {
-  if (d.ctrl->err) return;
+  __shared__ ClassTable tab;
+  if (!stream_begin<CLS>(d, &tab)) return;
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -177,36 +176,21 @@ __global__ void __launch_bounds__(256, PD_MINB_QA) k_osb_a32q(DevBody d, int kst
     const float4 hi = d.uhi[self], lo = d.ulo[self];
     const float2 nhi = make_float2(-hi.x, -hi.y), nlo = make_float2(-lo.x, -lo.y);
     const float nhz = -hi.z, nlz = -lo.z;
-    const int* pn = d.nbr + sbase + lane;
-    const float4* pg = d.geo + sbase + lane;
-    unsigned* pw = d.bits + (sbase >> 5);
     KSum2 mt;
     KSum1 th;
     float dm = 0.f;
     int na = 0;
-    int nj0 = self, nj1 = self;
-    float4 ng0 = make_float4(0.f, 0.f, 0.f, 1.f), ng1 = ng0;
-    unsigned nw0 = 0u, nw1 = 0u;
-    // the state words are plain loads: this warp owns them and rewrites them below
-    auto load_pair = [&](int r) {
-      const bool two = r + 1 < rows;
-      nw0 = pw[r];
-      nw1 = two ? pw[r + 1] : 0u;
-      nj0 = ld_stream(pn + 32 * r);
-      ng0 = ld_stream(pg + 32 * r);
-      if (two) { nj1 = ld_stream(pn + 32 * r + 32); ng1 = ld_stream(pg + 32 * r + 32); }
-      else { nj1 = self; ng1 = make_float4(0.f, 0.f, 0.f, 1.f); }
-    };
-    if (rows > 0) load_pair(0);
+    Stream32<CLS, true> st(d, &tab, s, sbase, rows, lane, self);
     for (int r = 0; r < rows; r += 2) {
       const bool two = r + 1 < rows;
-      const unsigned w0 = nw0, w1 = nw1;
-      const bool a0 = (w0 >> lane) & 1u, a1 = (w1 >> lane) & 1u;
-      const int j0 = a0 ? nj0 : self, j1 = a1 ? nj1 : self;
-      const float4 g0 = ng0, g1 = ng1;
+      unsigned w0, w1;
+      bool a0, a1;
+      int j0, j1;
+      float4 g0, g1;
+      st.take(r, w0, w1, a0, a1, j0, j1, g0, g1);
       const float4 hj0 = __ldg(d.uhi + j0), lj0 = __ldg(d.ulo + j0);
       const float4 hj1 = __ldg(d.uhi + j1), lj1 = __ldg(d.ulo + j1);
-      if (r + 2 < rows) load_pair(r + 2);
+      if (r + 2 < rows) st.load(r + 2);
       bool act0, act1;
 #pragma unroll
       for (int u = 0; u < 2; u++) {
@@ -236,8 +220,8 @@ __global__ void __launch_bounds__(256, PD_MINB_QA) k_osb_a32q(DevBody d, int kst
       const unsigned c0 = __ballot_sync(0xffffffffu, act0);
       const unsigned c1 = __ballot_sync(0xffffffffu, act1);
       if (lane == 0) {
-        if (c0 != w0) pw[r] = c0;
-        if (two && c1 != w1) pw[r + 1] = c1;
+        if (c0 != w0) d.bits[(sbase >> 5) + r] = c0;
+        if (two && c1 != w1) d.bits[(sbase >> 5) + r + 1] = c1;
       }
     }
     if (valid) {
@@ -270,8 +254,10 @@ __global__ void __launch_bounds__(256, PD_MINB_QA) k_osb_a32q(DevBody d, int kst
 #ifndef PD_MINB_QBB
 #define PD_MINB_QBB 4
 #endif
+template <bool CLS>
 __global__ void __launch_bounds__(256, PD_MINB_QBB) k_bb32q(DevBody d, int kstep) {
-  if (d.ctrl->err) return;
+  __shared__ ClassTable tab;
+  if (!stream_begin<CLS>(d, &tab)) return;
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -286,35 +272,20 @@ __global__ void __launch_bounds__(256, PD_MINB_QBB) k_bb32q(DevBody d, int kstep
     const float4 hi = d.uhi[self], lo = d.ulo[self];
     const float2 nhi = make_float2(-hi.x, -hi.y), nlo = make_float2(-lo.x, -lo.y);
     const float nhz = -hi.z, nlz = -lo.z;
-    const int* pn = d.nbr + sbase + lane;
-    const float4* pg = d.geo + sbase + lane;
-    unsigned* pw = d.bits + (sbase >> 5);
     KSum2 bxy;
     KSum1 bz;
     int na = 0;
-    int nj0 = self, nj1 = self;
-    float4 ng0 = make_float4(0.f, 0.f, 0.f, 1.f), ng1 = ng0;
-    unsigned nw0 = 0u, nw1 = 0u;
-    // the state words are plain loads: this warp owns them and rewrites them below
-    auto load_pair = [&](int r) {
-      const bool two = r + 1 < rows;
-      nw0 = pw[r];
-      nw1 = two ? pw[r + 1] : 0u;
-      nj0 = ld_stream(pn + 32 * r);
-      ng0 = ld_stream(pg + 32 * r);
-      if (two) { nj1 = ld_stream(pn + 32 * r + 32); ng1 = ld_stream(pg + 32 * r + 32); }
-      else { nj1 = self; ng1 = make_float4(0.f, 0.f, 0.f, 1.f); }
-    };
-    if (rows > 0) load_pair(0);
+    Stream32<CLS, true> st(d, &tab, s, sbase, rows, lane, self);
     for (int r = 0; r < rows; r += 2) {
       const bool two = r + 1 < rows;
-      const unsigned w0 = nw0, w1 = nw1;
-      const bool a0 = (w0 >> lane) & 1u, a1 = (w1 >> lane) & 1u;
-      const int j0 = a0 ? nj0 : self, j1 = a1 ? nj1 : self;
-      const float4 g0 = ng0, g1 = ng1;
+      unsigned w0, w1;
+      bool a0, a1;
+      int j0, j1;
+      float4 g0, g1;
+      st.take(r, w0, w1, a0, a1, j0, j1, g0, g1);
       const float4 hj0 = __ldg(d.uhi + j0), lj0 = __ldg(d.ulo + j0);
       const float4 hj1 = __ldg(d.uhi + j1), lj1 = __ldg(d.ulo + j1);
-      if (r + 2 < rows) load_pair(r + 2);
+      if (r + 2 < rows) st.load(r + 2);
       bool act0, act1;
 #pragma unroll
       for (int u = 0; u < 2; u++) {
@@ -334,8 +305,8 @@ __global__ void __launch_bounds__(256, PD_MINB_QBB) k_bb32q(DevBody d, int kstep
       const unsigned c0 = __ballot_sync(0xffffffffu, act0);
       const unsigned c1 = __ballot_sync(0xffffffffu, act1);
       if (lane == 0) {
-        if (c0 != w0) pw[r] = c0;
-        if (two && c1 != w1) pw[r + 1] = c1;
+        if (c0 != w0) d.bits[(sbase >> 5) + r] = c0;
+        if (two && c1 != w1) d.bits[(sbase >> 5) + r + 1] = c1;
       }
     }
     if (valid) {
@@ -371,31 +342,36 @@ static int grid_pk(long long nslices, int block) {
   return (int)blocks;
 }
 
-int launch_force32_pk(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s) {
+template <bool CLS>
+static int launch_pk(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s) {
   const int grid = grid_pk(d.nslices, c.block);
   const bool lin = d.kernel == KER_LINEAR;
   int launches = 0;
   if (d.material == MAT_BB) {
     if (phase == 2) return 0;
-    k_bb32q<<<grid, c.block, 0, s>>>(d, kstep);
+    k_bb32q<CLS><<<grid, c.block, 0, s>>>(d, kstep);
     return 1;
   }
   if (phase != 2) {
     if (c.fullk) {
-      if (lin) k_osb_a32q<true, true><<<grid, c.block, 0, s>>>(d, kstep);
-      else k_osb_a32q<true, false><<<grid, c.block, 0, s>>>(d, kstep);
+      if (lin) k_osb_a32q<CLS, true, true><<<grid, c.block, 0, s>>>(d, kstep);
+      else k_osb_a32q<CLS, true, false><<<grid, c.block, 0, s>>>(d, kstep);
     } else {
-      if (lin) k_osb_a32q<false, true><<<grid, c.block, 0, s>>>(d, kstep);
-      else k_osb_a32q<false, false><<<grid, c.block, 0, s>>>(d, kstep);
+      if (lin) k_osb_a32q<CLS, false, true><<<grid, c.block, 0, s>>>(d, kstep);
+      else k_osb_a32q<CLS, false, false><<<grid, c.block, 0, s>>>(d, kstep);
     }
     launches++;
   }
   if (phase != 1) {
-    if (lin) k_osb_b32q<true><<<grid, c.block, 0, s>>>(d, kstep);
-    else k_osb_b32q<false><<<grid, c.block, 0, s>>>(d, kstep);
+    if (lin) k_osb_b32q<CLS, true><<<grid, c.block, 0, s>>>(d, kstep);
+    else k_osb_b32q<CLS, false><<<grid, c.block, 0, s>>>(d, kstep);
     launches++;
   }
   return launches;
+}
+
+int launch_force32_pk(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s) {
+  return d.ncls > 0 ? launch_pk<true>(d, c, kstep, phase, s) : launch_pk<false>(d, c, kstep, phase, s);
 }
 
 }  // namespace pd

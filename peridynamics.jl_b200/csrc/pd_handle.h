@@ -70,6 +70,7 @@ struct pd_handle {
   // FP32 OSB / CMat: the stored weighted volumes / shape tensors are stale (bond states
   // changed outside the kernels)
   bool kfull = true;
+  bool cls_tried = false;  // bond classes were looked for in the current layout
   bool damage_valid = false;
   bool has_bext_state = false;
   // boundary conditions (host side)

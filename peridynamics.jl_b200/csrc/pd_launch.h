@@ -88,6 +88,11 @@ void launch_split_u(const DevBody& d, cudaStream_t s);
 // the split of rows[0 .. n) (halo rows that received a displacement)
 void launch_split_u_rows(const DevBody& d, const int* rows, long long n, cudaStream_t s);
 
+// bond classes of an FP32 body with one lane per point (pd_classes.cu): *ncls = 0 when the bonds
+// fall into more than 256. The arrays are the caller's to free
+cudaError_t build_classes(const DevBody& d, long long nslots, unsigned** cls, float4** geo, int** dj,
+                          int* ncls, cudaStream_t s);
+
 // sliced bond layout and bond-array helpers (pd_layout.cu)
 cudaError_t build_slices(long long n, const long long* off, int G, long long** soff_out,
                          long long* nslices_out, long long* nslots_out, cudaStream_t s);
