@@ -141,6 +141,40 @@ static pd_status check_symmetry(pd_handle* h) {
   return PD_OK;
 }
 
+// FP32 bodies with one lane per point gather from tiles in shared memory and, on a regular lattice,
+// read a bond's geometry as one byte. Both are made once per layout; a body without tiles or
+// classes, or without the memory for them, runs the kernels that its bond-stream variant names.
+static pd_status ensure_tiles(pd_handle* h) {
+  if (h->tiles_tried || h->precision == PD_PREC_FP64 || !packed_supported(h->d, 1))
+    return PD_OK;
+  h->tiles_tried = true;
+  TileArrays t;
+  cudaError_t e = build_tiles(h->d, h->nslots, &t, h->stream);
+  if (e != cudaErrorMemoryAllocation) PD_CUDA(e);
+  else cudaGetLastError();
+  if (t.pt == nullptr) return PD_OK;
+  for (void* p : {(void*)t.pt, (void*)t.n, (void*)t.lidx, (void*)t.lown}) h->allocs.push_back(p);
+  h->d.tile_pt = t.pt;
+  h->d.tile_n = t.n;
+  h->d.lidx = t.lidx;
+  h->d.lown = t.lown;
+  h->d.tile_cap = t.cap;
+  h->version++;
+  unsigned* cls = nullptr;
+  float4* geo = nullptr;
+  int ncls = 0;
+  e = build_classes(h->d, h->nslots, &cls, &geo, &ncls, h->stream);
+  if (e != cudaErrorMemoryAllocation) PD_CUDA(e);
+  else cudaGetLastError();
+  if (ncls == 0) return PD_OK;
+  h->allocs.push_back(cls);
+  h->allocs.push_back(geo);
+  h->d.cls = cls;
+  h->d.cls_geo = geo;
+  h->d.ncls = ncls;
+  return PD_OK;
+}
+
 // CSR bond lists (device) -> sliced layout with one lane per point, bond geometry, reverse
 // positions, all bonds active; then the point state.
 static pd_status finish_create(pd_handle* h, int* dnbr_csr, const double* dL, const unsigned char* dfp) {
@@ -160,7 +194,14 @@ static pd_status finish_create(pd_handle* h, int* dnbr_csr, const double* dL, co
   }
   long long* soff = nullptr;
   long long ns = 0, nslots = 0;
-  PD_CUDA(build_slices(n, h->d.off, 1, &soff, &ns, &nslots, h->stream));
+  if (h->precision != PD_PREC_FP64) {
+    PD_CUDA(build_places(h->d, h->grid, &h->pt, &h->place, h->stream));
+    h->allocs.push_back(h->pt);
+    h->allocs.push_back(h->place);
+    h->d.pt = h->pt;
+    h->d.place = h->place;
+  }
+  PD_CUDA(build_slices(n, h->d.off, h->d.pt, 1, &soff, &ns, &nslots, h->stream));
   h->allocs.push_back(soff);
   h->d.soff = soff;
   h->d.nslices = ns;
@@ -262,6 +303,7 @@ static pd_status finish_create(pd_handle* h, int* dnbr_csr, const double* dL, co
   launch_count_active(h->d, h->stream);
   PD_CUDA(cudaGetLastError());
   PD_TRY(check_symmetry(h));
+  PD_TRY(ensure_tiles(h));
   PD_CUDA(cudaStreamSynchronize(h->stream));
   return PD_OK;
 }
@@ -273,7 +315,9 @@ static pd_status relayout(pd_handle* h, int G) {
   DevBody a = h->d, b = h->d;
   long long* soff = nullptr;
   long long ns = 0, nslots = 0;
-  PD_CUDA(build_slices(h->n, h->d.off, G, &soff, &ns, &nslots, h->stream));
+  b.pt = G == 1 ? h->pt : nullptr;
+  b.place = G == 1 ? h->place : nullptr;
+  PD_CUDA(build_slices(h->n, h->d.off, b.pt, G, &soff, &ns, &nslots, h->stream));
   h->allocs.push_back(soff);
   b.soff = soff;
   b.nslices = ns;
@@ -331,45 +375,46 @@ static pd_status relayout(pd_handle* h, int G) {
   dfree(h, (void*)a.soff); dfree(h, (void*)a.nbr); dfree(h, (void*)a.rev);
   dfree(h, (void*)a.len64); dfree(h, (void*)a.geo); dfree(h, a.bits);
   dfree(h, (void*)a.sc64); dfree(h, (void*)a.sc32);
-  dfree(h, (void*)a.cls); dfree(h, (void*)a.cls_geo); dfree(h, (void*)a.cls_dj);
+  for (const void* p : {(const void*)a.tile_pt, (const void*)a.tile_n, (const void*)a.lidx,
+                        (const void*)a.lown, (const void*)a.cls, (const void*)a.cls_geo})
+    dfree(h, const_cast<void*>(p));
+  b.tile_pt = nullptr;
+  b.tile_n = nullptr;
+  b.lidx = nullptr;
+  b.lown = nullptr;
   b.cls = nullptr;
   b.cls_geo = nullptr;
-  b.cls_dj = nullptr;
   b.ncls = 0;
-  h->cls_tried = false;
+  h->tiles_tried = false;
   h->d = b;
   h->nslots = nslots;
   destroy_graph(h);
-  return PD_OK;
+  return ensure_tiles(h);
 }
 
-// The packed FP32 kernels (pipe 5) read the bonds of a body on a regular lattice as one byte each.
-// Looked for once per layout, when the variant is chosen (two passes over the bonds); a body
-// without classes, or without the memory for them, keeps the full bond stream.
-static pd_status ensure_classes(pd_handle* h) {
-  if (h->cls_tried || h->precision == PD_PREC_FP64 || h->cfg.pipe != 5 || !packed_supported(h->d, 1))
-    return PD_OK;
-  h->cls_tried = true;
-  unsigned* cls = nullptr;
-  float4* geo = nullptr;
-  int* dj = nullptr;
-  int ncls = 0;
-  const cudaError_t e = build_classes(h->d, h->nslots, &cls, &geo, &dj, &ncls, h->stream);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    return PD_OK;
+// The lattice that the places of the points are laid out on: the bounding box's corner, the spacing
+// that the mean volume implies, and first the axis on which consecutive points lie (of the first
+// few thousand). Only the speed of the kernels depends on how well it fits the body.
+static PlaceGrid place_grid(long long n, const double* X, const double* V) {
+  PlaceGrid g{};
+  double vol = 0;
+  int steps[3] = {0, 0, 0};
+  for (int a = 0; a < 3; a++) { g.lo[a] = n > 0 ? X[a] : 0.0; g.axis[a] = a; }
+  for (long long i = 0; i < n; i++) {
+    for (int a = 0; a < 3; a++) g.lo[a] = std::min(g.lo[a], X[3 * i + a]);
+    vol += V[i];
   }
-  PD_CUDA(e);
-  if (ncls == 0) return PD_OK;
-  h->allocs.push_back(cls);
-  h->allocs.push_back(geo);
-  h->allocs.push_back(dj);
-  h->d.cls = cls;
-  h->d.cls_geo = geo;
-  h->d.cls_dj = dj;
-  h->d.ncls = ncls;
-  h->version++;
-  return PD_OK;
+  for (long long i = 1; i < std::min<long long>(n, 4096); i++) {
+    int m = 0;
+    for (int a = 1; a < 3; a++)
+      if (std::fabs(X[3 * i + a] - X[3 * i - 3 + a]) > std::fabs(X[3 * i + m] - X[3 * i - 3 + m])) m = a;
+    steps[m]++;
+  }
+  const int first = (int)(std::max_element(steps, steps + 3) - steps);
+  std::swap(g.axis[0], g.axis[first]);
+  const double h = n > 0 ? std::cbrt(vol / n) : 1.0;
+  g.inv = h > 0 && std::isfinite(h) ? 1.0 / h : 1.0;
+  return g;
 }
 
 static pd_status begin_create(const pd_body_desc* desc, pd_handle** out, pd_handle** hp) {
@@ -408,6 +453,7 @@ static pd_status begin_create(const pd_body_desc* desc, pd_handle** out, pd_hand
                          desc->volume[i]);
     cur[i] = h->precision == PD_PREC_FP64 ? X0[i] : make_double4(0, 0, 0, desc->volume[i]);
   }
+  h->grid = place_grid(n, desc->position, desc->volume);
   double4 *dX0 = nullptr, *dcur = nullptr;
   PD_TRY(dalloc(h, &dX0, n));
   PD_TRY(dalloc(h, &dcur, n));
@@ -1421,7 +1467,6 @@ extern "C" pd_status pd_autotune(pd_handle* h, int32_t* group_out, int32_t* bloc
   std::vector<Cand> cands;
   // five evaluations of the current configuration after one warm-up
   auto time_cfg = [&](float* out) -> pd_status {
-    PD_TRY(ensure_classes(h));
     launch_force(h, 0, 0);
     cudaEventRecord(e0, h->stream);
     for (int r = 0; r < 5; r++) launch_force(h, 0, 0);
@@ -1479,7 +1524,6 @@ extern "C" pd_status pd_autotune(pd_handle* h, int32_t* group_out, int32_t* bloc
     if (c.ms < best) { best = c.ms; bestc = c.c; }
   PD_TRY(relayout(h, bestc.group));
   h->cfg = bestc;
-  PD_TRY(ensure_classes(h));
   destroy_graph(h);
   if (group_out) *group_out = bestc.group;
   if (block_out) *block_out = bestc.block;
@@ -1603,10 +1647,9 @@ extern "C" pd_status pd_set_pipeline(pd_handle* h, int32_t pipe) {
     return fail(PD_ERR_ARG, "the packed-pair kernels are FP32 ones");
   if (pipe >= 1 && pipe <= 3 && (h->precision != PD_PREC_FP32_KAHAN || !tma_supported(h->d)))
     return fail(PD_ERR_ARG, "the staged bond stream needs the FP32 path, one lane per point and BB or OSB");
-  PD_CUDA(cudaSetDevice(h->device));
   h->cfg.pipe = pipe;
   destroy_graph(h);
-  return ensure_classes(h);
+  return PD_OK;
 }
 
 // helpers shared with pd_nk.cu

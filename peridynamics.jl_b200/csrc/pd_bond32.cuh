@@ -1,0 +1,215 @@
+// pd_bond32.cuh -- the per-bond arithmetic of the packed FP32 kernels: the x and y components of
+// every vector are one packed pair, z is scalar. Shared by the kernels that gather from global
+// memory (pd_force32_pk.cu, pd_force32.cu) and from a tile in shared memory (pd_tile32.cu): a body's
+// results do not depend on which of them runs.
+#pragma once
+#include "pd_common.cuh"
+#include "pd_pack.cuh"
+
+namespace pd {
+namespace pack {
+
+// Rows whose terms are summed from zero before they join the total of a point: a slice's rows may be
+// shared among warps (pd_tile32.cu) without a change in the sums.
+constexpr int SEG32 = 16;
+
+// A segment's compensated sum joins the total's, in the form whose low part is below half a unit of
+// the high one: rows of padding at its end (there are as many as the longest list of the slice
+// asks for) leave that form as it is.
+__device__ __forceinline__ void join(KSum1& t, const KSum1& s) {
+  const float v = s.s + s.n;
+  t.add(v);
+  t.n += (s.s - v) + s.n;
+}
+__device__ __forceinline__ void join(KSum2& t, const KSum2& s) {
+  const float2 v = add2(s.s, s.n);
+  t.add(v);
+  t.n = add2(t.n, add2(sub2(s.s, v), s.n));
+}
+
+// the own point's displacement, negated
+struct Own32 {
+  float2 nhi, nlo;
+  float nhz, nlz;
+  __device__ __forceinline__ Own32(const float4& hi, const float4& lo)
+      : nhi(make_float2(-hi.x, -hi.y)), nlo(make_float2(-lo.x, -lo.y)), nhz(-hi.z), nlz(-lo.z) {}
+};
+
+// 1 / L of a bond
+__device__ __forceinline__ float bond_rl(float w) { return __fdividef(1.f, fabsf(w)); }
+
+// du = (h_j - h_i) + (l_j - l_i) and num = l^2 - L^2 = 2 xi . du + du . du: the two products apart,
+// since the sum 2 xi + du would round xi's share of a small du
+__device__ __forceinline__ void bond_du(const float4& g, const float4& hj, const float4& lj,
+                                        const Own32& o, float2& dxy, float& dz, float& num) {
+  dxy = add2(add2(xy(hj), o.nhi), add2(xy(lj), o.nlo));
+  dz = (hj.z + o.nhz) + (lj.z + o.nlz);
+  const float2 gd = mul2(xy(g), dxy), d2 = mul2(dxy, dxy);
+  num = fmaf(2.f, fmaf(g.z, dz, gd.x + gd.y), fmaf(dz, dz, d2.x + d2.y));
+}
+
+// eta = xi + du, rl = 1 / |eta|, e = l - L = num / (l + L) without the cancellation of l - L
+struct BondP {
+  float2 exy;
+  float ez;
+  float rl, L, e;
+};
+
+__device__ __forceinline__ void bond_pk(const float4& g, const float4& hj, const float4& lj,
+                                        const Own32& o, BondP& B) {
+  float2 dxy;
+  float dz, num;
+  bond_du(g, hj, lj, o, dxy, dz, num);
+  B.exy = add2(xy(g), dxy);
+  B.ez = g.z + dz;
+  const float2 e2 = mul2(B.exy, B.exy);
+  const float l2 = fmaf(B.ez, B.ez, e2.x + e2.y);
+  B.rl = rsqrtf(l2);
+  B.L = fabsf(g.w);
+  B.e = __fdividef(num, fmaf(l2, B.rl, B.L));
+}
+
+// influence function; LIN: the linear one, delta / L
+template <bool LIN>
+__device__ __forceinline__ float omega_pk(int kernel, float delta, float L, float rL) {
+  if constexpr (LIN) return delta * rL;
+  else return kernel == KER_LINEAR ? delta * rL : omega_of_f(kernel, delta, L);
+}
+
+// the failure test of CriticalStretch
+__device__ __forceinline__ bool stays(bool a, float eps, float epsc, float w) {
+  return a && !(eps > epsc && w > 0.f);
+}
+
+// omega L V e of a bond, the dilatation's term; LIN: without the factor delta, which leaves the sum
+template <bool LIN>
+__device__ __forceinline__ float dil_term(int kernel, float delta, const BondP& B, float rL, float V) {
+  if constexpr (LIN) return V * B.e;
+  else return omega_pk<LIN>(kernel, delta, B.L, rL) * V * B.L * B.e;
+}
+
+// omega V xi^2, the weighted volume's term
+template <bool LIN>
+__device__ __forceinline__ float vol_term(int kernel, float delta, const float4& g, float rL, float V) {
+  const float2 g2 = mul2(xy(g), xy(g));
+  return omega_pk<LIN>(kernel, delta, fabsf(g.w), rL) * V * fmaf(g.z, g.z, g2.x + g2.y);
+}
+
+// OSB: omega ((c2_i + c2_j) L + (c1_i + c1_j) e) V / l; LIN: without the factor delta
+template <bool LIN>
+__device__ __forceinline__ float osb_pair(int kernel, float delta, const BondP& B, float rL, float2 cs,
+                                          float V) {
+  const float f = LIN ? fmaf(cs.x, B.e * rL, cs.y)
+                      : omega_of_f(kernel, delta, B.L) * fmaf(cs.y, B.L, cs.x * B.e);
+  return f * (V * B.rl);
+}
+
+// OSB: {c1, c2} and the dilatation of a point from its weighted volume w and the sum t of the
+// dilatation's terms. In double: a factor rounded here moves all of the point's bonds the same way
+// (relative error of the forces against 64 bits, 975-point coupon: 9.2e-8 in float, 8.0e-8 so).
+template <bool LIN>
+__device__ __forceinline__ float2 osb_point(const DevParam& P, float w, float t, float& dil) {
+  dil = 0.f;
+  if (w == 0.f) return make_float2(0.f, 0.f);
+  const double rw = 1.0 / (double)w;
+  const double th = 3.0 * rw * (LIN ? P.delta * (double)t : (double)t);
+  dil = (float)th;
+  return make_float2((float)(15.0 * P.G * rw), (float)(th * (3.0 * P.K - 5.0 * P.G) * rw));
+}
+
+// the force on a point: its sum times the factor f that all bonds share (in double, as above)
+__device__ __forceinline__ void store_force(const DevBody& d, long long i, int kstep, double f,
+                                            const float2 v, float vz) {
+  const float x = (float)(f * (double)v.x), y = (float)(f * (double)v.y), z = (float)(f * (double)vz);
+  d.b32[3 * i] = x;
+  d.b32[3 * i + 1] = y;
+  d.b32[3 * i + 2] = z;
+  if (isnan(x) || isnan(y) || isnan(z)) {
+    const long long step = d.ctrl->base + kstep;
+    if (atomicExch(&d.ctrl->err, 1) == 0) d.ctrl->err_step = step;
+    else atomicMin(&d.ctrl->err_step, step);
+  }
+}
+
+// correspondence phase A: the constants of a point
+struct CorrA {
+  float epsc, thr, ks, delta;
+  // ks: a bond's weight in the sums with xi and du over the horizon, omega V / delta^5; with the
+  // linear influence function delta / L, V / (L delta^4). thr: l^2 - L^2 below this share of L^2 is
+  // a stretch below eps_c whatever the rounding
+  __device__ __forceinline__ CorrA(const DevParam& P, bool lin) : epsc(P.epscf), delta(P.deltaf) {
+    const float w = P.vscale * P.inv_delta * P.inv_delta;
+    ks = lin ? delta * w : w;
+    thr = epsc > 0.f ? (2.f * epsc + epsc * epsc) * (1.f - 1e-5f) : -INFINITY;
+  }
+};
+
+// whether an active bond stays: the test on eps = (l - L) / L only for those beyond thr
+__device__ __forceinline__ bool corr_stays(bool a, const CorrA& c, const float4& g, float rL,
+                                           const float2 dxy, float dz, float num) {
+  if (!a || !(g.w > 0.f) || num < c.thr * (g.w * g.w)) return a;
+  const float2 e = add2(xy(g), dxy);
+  const float ez = g.z + dz;
+  const float2 e2 = mul2(e, e);
+  const float l2 = fmaf(ez, ez, e2.x + e2.y);
+  return !(__fdividef(num, fmaf(l2, rsqrtf(l2), g.w)) * rL > c.epsc);
+}
+
+template <bool LIN>
+__device__ __forceinline__ float corr_weight(int kernel, const CorrA& c, const float4& g, float rL, float V) {
+  return (LIN ? rL : omega_of_f(kernel, c.delta, fabsf(g.w))) * V * c.ks;
+}
+
+// the sums of correspondence phase A: the displacement gradient (rows x, y of every column packed;
+// plain FP32 sums: compensated ones moved the displacement after 250 steps by less than the error
+// of the form) and, in full, the shape tensor {xx, yy, zz, xy, xz, yz} (compensated)
+template <bool FULLK>
+struct CorrSums {
+  float2 Hxy[3];
+  float Hz[3];
+  KSum2 K01, K23, K45;
+  float dK[6];
+  __device__ __forceinline__ CorrSums() {
+#pragma unroll
+    for (int c = 0; c < 3; c++) { Hxy[c] = both(0.f); Hz[c] = 0.f; }
+#pragma unroll
+    for (int q = 0; q < 6; q++) dK[q] = 0.f;
+  }
+  __device__ __forceinline__ void add(float t, const float4& g, const float2 dxy, float dz) {
+    const float2 tX = mul2(both(t), xy(g));
+    const float tXz = t * g.z;
+    Hxy[0] = fma2(both(tX.x), dxy, Hxy[0]); Hz[0] = fmaf(tX.x, dz, Hz[0]);
+    Hxy[1] = fma2(both(tX.y), dxy, Hxy[1]); Hz[1] = fmaf(tX.y, dz, Hz[1]);
+    Hxy[2] = fma2(both(tXz), dxy, Hxy[2]);  Hz[2] = fmaf(tXz, dz, Hz[2]);
+    if constexpr (FULLK) {
+      K01.add(mul2(tX, xy(g)));
+      K23.add(make_float2(tXz * g.z, tX.x * g.y));
+      K45.add(mul2(tX, both(g.z)));
+    }
+  }
+  // a bond breaks: its term leaves the stored shape tensor
+  __device__ __forceinline__ void drop(float t, const float4& g) {
+    dK[0] += t * g.x * g.x; dK[1] += t * g.y * g.y; dK[2] += t * g.z * g.z;
+    dK[3] += t * g.x * g.y; dK[4] += t * g.x * g.z; dK[5] += t * g.y * g.z;
+  }
+};
+
+// correspondence phase B: V omega ((A_i + A_j) xi + (beta_i + beta_j) du), A column-major in
+// {a.x .. a.w, b.x .. b.w, c.x}, beta in c.y; LIN: without the factor delta
+__device__ __forceinline__ void corr_pair(const float4& g, const float2 dxy, float dz, const float4& ia,
+                                          const float4& ib, const float2& ic, const float4& ja,
+                                          const float4& jb, const float2& jc, float2& txy, float& tz) {
+  const float2 S01 = add2(make_float2(ia.x, ia.y), make_float2(ja.x, ja.y));
+  const float2 S23 = add2(make_float2(ia.z, ia.w), make_float2(ja.z, ja.w));
+  const float2 S45 = add2(make_float2(ib.x, ib.y), make_float2(jb.x, jb.y));
+  const float2 S67 = add2(make_float2(ib.z, ib.w), make_float2(jb.z, jb.w));
+  const float2 S8b = add2(ic, jc);
+  txy = mul2(both(S8b.y), dxy);
+  txy = fma2(S01, both(g.x), txy);
+  txy = fma2(make_float2(S23.y, S45.x), both(g.y), txy);
+  txy = fma2(S67, both(g.z), txy);
+  tz = fmaf(S23.x, g.x, fmaf(S45.y, g.y, fmaf(S8b.x, g.z, S8b.y * dz)));
+}
+
+}  // namespace pack
+}  // namespace pd

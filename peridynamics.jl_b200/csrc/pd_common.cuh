@@ -5,7 +5,8 @@
 //   off      int64[n+1]   n_neighbors of point i is off[i+1] - off[i] (the reference's CSR
 //                         order: bond k of point i is bond off[i] + k of the reference)
 //   Bond arrays are stored in a sliced layout with G lanes per point ("SELL"): the points
-//   are cut into slices of P = 32 / G consecutive points; slice s owns rows
+//   are cut into slices of P = 32 / G points (consecutive ones; FP32 with one lane per point: compact
+//   parts of the body, pd_tiles.cu); slice s owns rows
 //   [soff[s] / 32, soff[s+1] / 32) of 32 bond slots; bond k of the point p of the slice sits
 //   in row k / G at lane p * G + k % G. A warp walks one slice row by row, so every
 //   bond-array load of a warp is one contiguous 128-byte (int32) or 512-byte (float4)
@@ -90,10 +91,21 @@ struct DevBody {
   const int* rev;    // revk
   const double* len64;
   const float4* geo;
-  // bond classes (pd_classes.cu): one byte a bond into tables of ncls entries; ncls = 0: none
+  // one lane per point, FP32: the points in the order of their places in the slices (place q is
+  // lane q % 32 of slice q / 32) and the inverse; null where the places are the points
+  const int* pt;
+  const int* place;
+  // tiles of eight slices (pd_tiles.cu), or null: the points of a tile and of all its bonds
+  // (ascending, tile_cap apart), their number, the place in that list of every bond's neighbour
+  // (four rows of 16 bits a lane) and of every point
+  const int* tile_pt;
+  const int* tile_n;
+  const uint2* lidx;
+  const unsigned short* lown;
+  int tile_cap;
+  // FP32 bond classes (pd_classes.cu): one byte a bond into ncls records; ncls = 0: none
   const unsigned* cls;
   const float4* cls_geo;
-  const int* cls_dj;
   int ncls;
   const double4* X0;
   double4* cur;
@@ -150,11 +162,17 @@ __device__ __forceinline__ float omega_of_f(int kernel, float delta, float L) {
   return 0.0f;
 }
 
+// the point at place q of the slices
+__device__ __forceinline__ long long point_at(const DevBody& d, long long q) {
+  return d.pt ? d.pt[q] : q;
+}
+
 // slot of bond k of point i in the sliced layout
 __device__ __forceinline__ long long bond_slot(const DevBody& d, long long i, int k) {
   const int G = d.lg, P = 32 / G;
-  const long long s = i / P;
-  const int p = (int)(i - s * P);
+  const long long q = d.place ? d.place[i] : i;
+  const long long s = q / P;
+  const int p = (int)(q - s * P);
   return d.soff[s] + (long long)(k / G) * 32 + p * G + (k % G);
 }
 
@@ -189,8 +207,9 @@ __device__ __forceinline__ void clear_bit(unsigned int* bits, long long b) {
 
 // point, slice rows and bond count of the lane
 #define PD_SLICE_SETUP                                                                      \
-  const long long i = s * PPW + sub;                                                        \
-  const bool valid = i < d.n;                                                               \
+  const long long place_ = s * PPW + sub;                                                   \
+  const bool valid = place_ < d.n;                                                          \
+  const long long i = valid ? point_at(d, place_) : place_;                                 \
   const long long sbase = d.soff[s];                                                        \
   const int rows = (int)((d.soff[s + 1] - sbase) >> 5);                                     \
   const int cnt = valid ? (int)(d.off[i + 1] - d.off[i]) : 0;

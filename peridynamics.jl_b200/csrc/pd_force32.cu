@@ -17,10 +17,11 @@
 // cancel) and a horizon-scaled shape tensor K' = K / delta^5 (the unscaled det K underflows
 // FP32 for millimetre lattices). The stress formulas are the reference's, rewritten in
 // terms of E = (H + H^T + H^T H) / 2 without cancelling subtractions.
+#include "pd_bond32.cuh"
 #include "pd_common.cuh"
 #include "pd_launch.h"
 #include "pd_pack.cuh"
-#include "pd_stream32.cuh"
+#include "pd_point32.cuh"
 
 namespace pd {
 
@@ -526,129 +527,9 @@ __global__ void __launch_bounds__(256, PD_MINB_UB) k_osb_b32u(DevBody d, int kst
   }
 }
 
-// ------------------------------------------------------------------------------------------
-// FP32 3x3 helpers (column-major) for the correspondence material
-// ------------------------------------------------------------------------------------------
-__device__ __forceinline__ void fcross(const float* a, const float* b, float* c) {
-  c[0] = a[1] * b[2] - a[2] * b[1];
-  c[1] = a[2] * b[0] - a[0] * b[2];
-  c[2] = a[0] * b[1] - a[1] * b[0];
-}
-__device__ __forceinline__ void finv3(const float* A, float* R) {
-  float x0[3] = {A[0], A[1], A[2]}, y0[3], y1[3], y2[3];
-  fcross(A + 3, A + 6, y0);
-  const float d = x0[0] * y0[0] + x0[1] * y0[1] + x0[2] * y0[2];
-  for (int k = 0; k < 3; k++) { x0[k] /= d; y0[k] /= d; }
-  fcross(A + 6, x0, y1);
-  fcross(x0, A + 3, y2);
-  for (int c = 0; c < 3; c++) { R[3 * c] = y0[c]; R[1 + 3 * c] = y1[c]; R[2 + 3 * c] = y2[c]; }
-}
-__device__ __forceinline__ void fmatmul(const float* A, const float* B, float* C) {
-  for (int r = 0; r < 3; r++)
-    for (int c = 0; c < 3; c++)
-      C[r + 3 * c] = A[r] * B[3 * c] + A[r + 3] * B[1 + 3 * c] + A[r + 6] * B[2 + 3 * c];
-}
-
-// P(F = I + H) of the reference's models, written without the cancelling F^T F - I
-__device__ void pk1_32(int cmodel, const DevParam& p, const float* H, float* P) {
-  float E[9], S[9], HS[9];
-  for (int r = 0; r < 3; r++)
-    for (int c = 0; c < 3; c++) {
-      const float hth = H[3 * r] * H[3 * c] + H[1 + 3 * r] * H[1 + 3 * c] + H[2 + 3 * r] * H[2 + 3 * c];
-      E[r + 3 * c] = 0.5f * (H[r + 3 * c] + H[c + 3 * r] + hth);
-    }
-  const float trE = E[0] + E[4] + E[8];
-  if (cmodel == CM_SVK) {
-    // S = lambda tr(E) I + 2 mu E
-    for (int k = 0; k < 9; k++) S[k] = 2.f * p.muf * E[k] + ((k % 4) == 0 ? p.lambdaf * trE : 0.f);
-  } else {
-    // J - 1 = tr H + (principal 2x2 minors of H) + det H
-    const float m2 = (H[0] * H[4] - H[3] * H[1]) + (H[0] * H[8] - H[6] * H[2]) + (H[4] * H[8] - H[7] * H[5]);
-    float dH;
-    {
-      float c[3];
-      fcross(H + 3, H + 6, c);
-      dH = H[0] * c[0] + H[1] * c[1] + H[2] * c[2];
-    }
-    const float jm1 = (H[0] + H[4] + H[8]) + m2 + dH;
-    const float J = 1.f + jm1;
-    float C[9], Ci[9], T[9];
-    for (int k = 0; k < 9; k++) C[k] = 2.f * E[k] + ((k % 4) == 0 ? 1.f : 0.f);
-    finv3(C, Ci);
-    if (cmodel == CM_NEOHOOKE) {
-      // S = mu (I - C^-1) + lambda ln J C^-1 = C^-1 (2 mu E + lambda ln J I)
-      const float lj = p.lambdaf * log1pf(jm1);
-      for (int k = 0; k < 9; k++) T[k] = 2.f * p.muf * E[k] + ((k % 4) == 0 ? lj : 0.f);
-    } else {
-      // NeoHookePenalty: S = C^-1 (2 G J^(-2/3) dev E + K/4 (J^2 - J^-2) I), P = 0 if J < eps
-      if (!(J >= 2.220446049250313e-16f)) {
-        for (int k = 0; k < 9; k++) P[k] = 0.f;
-        return;
-      }
-      const float jp = expf(-2.f / 3.f * log1pf(jm1));
-      const float iJ = 1.f / J;
-      const float vol = 0.25f * p.Kf * (jm1 * (J + 1.f) * iJ) * (J + iJ);
-      for (int k = 0; k < 9; k++)
-        T[k] = 2.f * p.Gf * jp * (E[k] - ((k % 4) == 0 ? trE / 3.f : 0.f)) + ((k % 4) == 0 ? vol : 0.f);
-    }
-    fmatmul(Ci, T, S);
-  }
-  // P = F S = S + H S
-  fmatmul(H, S, HS);
-  for (int k = 0; k < 9; k++) P[k] = S[k] + HS[k];
-}
-
 // -------------------------------------------------------------------------------------------
 // CMat phase A (correspondence.jl:193-224, 288-298; bond_system.jl:309-327)
 // -------------------------------------------------------------------------------------------
-// The phase-B state of a live point, from the scaled inverse shape tensor Kinv (the true
-// K^-1 = Kinv / delta^5), P K^-1 (scaled the same way) and H = F - I. The bond term
-// w (P K^-1 xi + S (dx - F xi)) is w (A xi + S du) with A = P K^-1 - S H, where S is the
-// stabilising stiffness: ZEMSilling beta I (c_force_density!, correspondence.jl:226-251; beta
-// in cst32), ZEMWan C : K^-1 (correspondence.jl:253-285, zem_stabilization.jl:32-42; the six
-// entries of the symmetric S in zw32, from the nonzero entries of the Hooke tensor: a = (1 - nu)
-// lambda / nu and lambda in the normal block, mu (both index orders) in the shear block).
-__device__ __forceinline__ void c_state_store32(const DevBody& d, const DevParam& P, long long i,
-                                                const float* PK, const float* Kinv, const float* H,
-                                                float id5) {
-  float A[9];
-  float4* cs = d.cst32 + 3 * i;
-  if (d.zem == ZEM_WAN) {
-    const float a = P.zwaf, l = P.lambdaf, m = P.muf;
-    const float S0 = (a * Kinv[0] + l * Kinv[4] + l * Kinv[8]) * id5;
-    const float S1 = (l * Kinv[0] + a * Kinv[4] + l * Kinv[8]) * id5;
-    const float S2 = (l * Kinv[0] + l * Kinv[4] + a * Kinv[8]) * id5;
-    const float S01 = m * (Kinv[3] + Kinv[1]) * id5;
-    const float S02 = m * (Kinv[6] + Kinv[2]) * id5;
-    const float S12 = m * (Kinv[7] + Kinv[5]) * id5;
-    const float Sm[9] = {S0, S01, S02, S01, S1, S12, S02, S12, S2};
-    float SH[9];
-    fmatmul(Sm, H, SH);
-#pragma unroll
-    for (int q = 0; q < 9; q++) A[q] = PK[q] * id5 - SH[q];
-    d.zw32[2 * i] = make_float4(S0, S1, S2, S01);
-    d.zw32[2 * i + 1] = make_float4(S02, S12, 0.f, 0.f);
-  } else {
-#pragma unroll
-    for (int q = 0; q < 9; q++) A[q] = PK[q] * id5 - P.betaf * H[q];
-  }
-  cs[0] = make_float4(A[0], A[1], A[2], A[3]);
-  cs[1] = make_float4(A[4], A[5], A[6], A[7]);
-  cs[2] = make_float4(A[8], d.zem == ZEM_WAN ? 0.f : P.betaf, 0.f, 0.f);
-}
-
-// a killed point's phase-B state: no term of its own, none for its neighbours
-__device__ __forceinline__ void c_state_clear32(const DevBody& d, long long i) {
-  float4* cs = d.cst32 + 3 * i;
-  cs[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-  cs[1] = make_float4(0.f, 0.f, 0.f, 0.f);
-  cs[2] = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (d.zem == ZEM_WAN) {
-    d.zw32[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    d.zw32[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-}
-
 // the correspondence phase A keeps 15 compensated 3x3 sums per point: it gets its own
 // occupancy bound (PD_MINB_CA resident blocks per SM). Measured on the 1M-point CMat block:
 // 1.50 / 1.44 / 1.49 ms at 2 / 3 / 4 blocks (109 / 80 / 64 registers).
@@ -921,43 +802,17 @@ __global__ void __launch_bounds__(256, PD_MINB_CB) k_c_b32(DevBody d, int kstep)
 #define PD_MINB_CQB 3
 #endif
 
-struct BondC {
-  float2 dxy;   // displacement difference, x and y
-  float dz;
-  float L, rL, eps;
-};
-
-__device__ __forceinline__ void bond_c(const float4& g, const float4& hj, const float4& lj,
-                                       const float2 nhi, const float nhz, const float2 nlo,
-                                       const float nlz, BondC& B) {
-  using namespace pack;
-  B.dxy = add2(add2(xy(hj), nhi), add2(xy(lj), nlo));
-  B.dz = (hj.z + nhz) + (lj.z + nlz);
-  const float2 exy = add2(xy(g), B.dxy);
-  const float ez = g.z + B.dz;
-  const float2 e2 = mul2(exy, exy);
-  const float l2 = fmaf(ez, ez, e2.x + e2.y);
-  const float l = l2 * rsqrtf(l2);
-  const float2 gd = mul2(xy(g), B.dxy);
-  const float xd = fmaf(g.z, B.dz, gd.x + gd.y);
-  const float2 d2 = mul2(B.dxy, B.dxy);
-  const float dd = fmaf(B.dz, B.dz, d2.x + d2.y);
-  B.L = fabsf(g.w);
-  B.rL = __fdividef(1.f, B.L);
-  B.eps = __fdividef(fmaf(2.f, xd, dd), l + B.L) * B.rL;
-}
-
-template <bool CLS, bool FULLK, bool LIN>
+template <bool FULLK, bool LIN>
 __global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kstep) {
   using namespace pack;
-  __shared__ ClassTable tab;
-  if (!stream_begin<CLS>(d, &tab)) return;
+  if (d.ctrl->err) return;
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long s = warp0; s < d.nslices; s += nwarps) {
-    const long long i = s * 32 + lane;
-    const bool valid = i < d.n;
+    const long long place = s * 32 + lane;
+    const bool valid = place < d.n;
+    const long long i = valid ? point_at(d, place) : place;
     const int self = valid ? (int)i : 0;
     const long long sbase = d.soff[s];
     const int rows = (int)((d.soff[s + 1] - sbase) >> 5);
@@ -965,158 +820,118 @@ __global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kste
     const unsigned meta = valid ? d.meta[i] : 0u;
     const DevParam& P = d.params[meta & META_PID_MASK];
     const float4 hi = d.uhi[self], lo = d.ulo[self];
-    const float2 nhi = make_float2(-hi.x, -hi.y), nlo = make_float2(-lo.x, -lo.y);
-    const float nhz = -hi.z, nlz = -lo.z;
-    const float epsc = P.epscf, id = P.inv_delta, vs = P.vscale;
-    const float2 id2 = make_float2(id, id);
-    KSum2 K01, K23, K45;        // FULLK: (xx, yy), (zz, xy), (xz, yz)
-    // rows x, y of column c of the displacement-gradient sum, and row z: plain FP32 sums (with
-    // compensated sums phase A took 0.648 against 0.594 ms on the 1M-point CMat block, and the
-    // FP32 displacement after 250 steps was within 1.33e-7 of FP64 against 1.37e-7 here, RMS
-    // 7.85e-8 both: the error of the form comes from elsewhere)
-    float2 Hxy[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-    float Hz[3] = {0.f, 0.f, 0.f};
-    float dK[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const Own32 own(hi, lo);
+    const CorrA cp(P, LIN);
+    const int* pn = d.nbr + sbase + lane;
+    const float4* pg = d.geo + sbase + lane;
+    unsigned* pw = d.bits + (sbase >> 5);
+    CorrSums<FULLK> S;
     int na = 0;
-    Stream32<CLS, true> st(d, &tab, s, sbase, rows, lane, self);
+    int nj0 = self, nj1 = self;
+    float4 ng0 = make_float4(0.f, 0.f, 0.f, 1.f), ng1 = ng0;
+    unsigned nw0 = 0u, nw1 = 0u;
+    auto load_pair = [&](int r) {
+      const bool two = r + 1 < rows;
+      nw0 = pw[r];
+      nw1 = two ? pw[r + 1] : 0u;
+      nj0 = ld_stream(pn + 32 * r);
+      ng0 = ld_stream(pg + 32 * r);
+      if (two) { nj1 = ld_stream(pn + 32 * r + 32); ng1 = ld_stream(pg + 32 * r + 32); }
+      else { nj1 = self; ng1 = make_float4(0.f, 0.f, 0.f, 1.f); }
+    };
+    if (rows > 0) load_pair(0);
     for (int r = 0; r < rows; r += 2) {
       const bool two = r + 1 < rows;
-      unsigned w0, w1;
-      bool a0, a1;
-      int j0, j1;
-      float4 g0, g1;
-      st.take(r, w0, w1, a0, a1, j0, j1, g0, g1);
+      const unsigned w0 = nw0, w1 = nw1;
+      const bool a0 = (w0 >> lane) & 1u, a1 = (w1 >> lane) & 1u;
+      const int j0 = a0 ? nj0 : self, j1 = a1 ? nj1 : self;
+      const float4 g0 = ng0, g1 = ng1;
       const float4 hj0 = __ldg(d.uhi + j0), lj0 = __ldg(d.ulo + j0);
       const float4 hj1 = __ldg(d.uhi + j1), lj1 = __ldg(d.ulo + j1);
-      if (r + 2 < rows) st.load(r + 2);
+      if (r + 2 < rows) load_pair(r + 2);
       bool act0, act1;
 #pragma unroll
       for (int u = 0; u < 2; u++) {
         const float4& g = u ? g1 : g0;
         const float4& hj = u ? hj1 : hj0;
         const bool a = u ? a1 : a0;
-        BondC B;
-        bond_c(g, hj, u ? lj1 : lj0, nhi, nhz, nlo, nlz, B);
-        const bool act = a && !(B.eps > epsc && g.w > 0.f);
-        const float om = omega_t<LIN>(d.kernel, P.deltaf, B.L, B.rL) * hj.w * vs;
-        const float t = act ? om : 0.f;
-        const float2 X = mul2(xy(g), id2);
-        const float Xz = g.z * id;
-        const float2 tU = mul2(make_float2(t, t), mul2(B.dxy, id2));
-        const float tUz = t * (B.dz * id);
-        Hxy[0] = add2(Hxy[0], mul2(tU, make_float2(X.x, X.x))); Hz[0] += tUz * X.x;
-        Hxy[1] = add2(Hxy[1], mul2(tU, make_float2(X.y, X.y))); Hz[1] += tUz * X.y;
-        Hxy[2] = add2(Hxy[2], mul2(tU, make_float2(Xz, Xz)));   Hz[2] += tUz * Xz;
-        if constexpr (FULLK) {
-          const float2 tX = mul2(make_float2(t, t), X);
-          const float tXz = t * Xz;
-          K01.add(mul2(tX, X));
-          K23.add(make_float2(tXz * Xz, tX.x * X.y));
-          K45.add(mul2(tX, make_float2(Xz, Xz)));
-        } else if (a && !act) {
-          // the bond breaks now: its term leaves the stored shape tensor
-          dK[0] += om * X.x * X.x; dK[1] += om * X.y * X.y; dK[2] += om * Xz * Xz;
-          dK[3] += om * X.x * X.y; dK[4] += om * X.x * Xz; dK[5] += om * X.y * Xz;
-        }
+        float2 dxy;
+        float dz, num;
+        bond_du(g, hj, u ? lj1 : lj0, own, dxy, dz, num);
+        const float rL = bond_rl(g.w);
+        const bool act = corr_stays(a, cp, g, rL, dxy, dz, num);
+        const float t = corr_weight<LIN>(d.kernel, cp, g, rL, hj.w);
+        S.add(act ? t : 0.f, g, dxy, dz);
+        if (!FULLK && a && !act) S.drop(t, g);
         if (u) act1 = act; else act0 = act;
       }
       na += (int)act0 + (int)act1;
       const unsigned c0 = __ballot_sync(0xffffffffu, act0);
       const unsigned c1 = __ballot_sync(0xffffffffu, act1);
       if (lane == 0) {
-        if (c0 != w0) d.bits[(sbase >> 5) + r] = c0;
-        if (two && c1 != w1) d.bits[(sbase >> 5) + r + 1] = c1;
+        if (c0 != w0) pw[r] = c0;
+        if (two && c1 != w1) pw[r + 1] = c1;
       }
     }
-    bool killed = false;
-    if (valid) {
-      float k6[6];
-      float2* ks = reinterpret_cast<float2*>(d.K32 + 6 * i);
-      if constexpr (FULLK) {
-        const float2 v01 = K01.value(), v23 = K23.value(), v45 = K45.value();
-        k6[0] = v01.x; k6[1] = v01.y; k6[2] = v23.x; k6[3] = v23.y; k6[4] = v45.x; k6[5] = v45.y;
-        ks[0] = make_float2(k6[0], k6[1]); ks[1] = make_float2(k6[2], k6[3]); ks[2] = make_float2(k6[4], k6[5]);
-      } else {
-        const float2 b0 = ks[0], b1 = ks[1], b2 = ks[2];
-        k6[0] = b0.x; k6[1] = b0.y; k6[2] = b1.x; k6[3] = b1.y; k6[4] = b2.x; k6[5] = b2.y;
-        if (dK[0] != 0.f || dK[1] != 0.f || dK[2] != 0.f) {  // a bond broke
-#pragma unroll
-          for (int q = 0; q < 6; q++) k6[q] -= dK[q];
-          ks[0] = make_float2(k6[0], k6[1]); ks[1] = make_float2(k6[2], k6[3]); ks[2] = make_float2(k6[4], k6[5]);
-        }
-      }
-      const float Km[9] = {k6[0], k6[3], k6[4],
-                           k6[3], k6[1], k6[5],
-                           k6[4], k6[5], k6[2]};
-      float Kinv[9], Hm[9], H[9];
-      finv3(Km, Kinv);
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        Hm[3 * c] = Hxy[c].x; Hm[3 * c + 1] = Hxy[c].y; Hm[3 * c + 2] = Hz[c];
-      }
-      fmatmul(Hm, Kinv, H);
-      bool hasnan = false;
-      for (int q = 0; q < 9; q++) { d.H32[9 * i + q] = H[q]; hasnan |= isnan(H[q]); }
-      const double damage = 1.0 - (double)na / (double)cnt;
-      killed = (meta & META_KILLED) || (!(meta & META_HALO) && (damage > d.maxdmg || hasnan));
-      if (killed) {
-        if (!(meta & META_KILLED)) d.meta[i] = meta | META_KILLED;
-        na = 0;
-        c_state_clear32(d, i);
-      } else {
-        float Pm[9], PK[9];
-        pk1_32(d.cmodel, P, H, Pm);
-        fmatmul(Pm, Kinv, PK);
-        c_state_store32(d, P, i, PK, Kinv, H, id * id * id * id * id);
-      }
-      d.n_active[i] = na;
-    }
+    const bool killed = valid && corr_point32<FULLK>(d, P, i, meta, cnt, na, S);
     if (!d.sym) {
       // directed bond states: a killed point loses all its bonds (correspondence.jl:293)
-      const unsigned kill_mask = __ballot_sync(0xffffffffu, valid && killed);
+      const unsigned kill_mask = __ballot_sync(0xffffffffu, killed);
       if (kill_mask && lane == 0)
         for (int r = 0; r < rows; r++) d.bits[(sbase >> 5) + r] &= ~kill_mask;
     }
   }
 }
 
-template <bool CLS, bool LIN>
+template <bool LIN>
 __global__ void __launch_bounds__(256, PD_MINB_CQB) k_c_b32q(DevBody d, int kstep) {
   using namespace pack;
-  __shared__ ClassTable tab;
-  if (!stream_begin<CLS>(d, &tab)) return;
+  if (d.ctrl->err) return;
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long s = warp0; s < d.nslices; s += nwarps) {
-    const long long i = s * 32 + lane;
-    const bool valid = i < d.n;
+    const long long place = s * 32 + lane;
+    const bool valid = place < d.n;
+    const long long i = valid ? point_at(d, place) : place;
     const int self = valid ? (int)i : 0;
     const long long sbase = d.soff[s];
     const int rows = (int)((d.soff[s + 1] - sbase) >> 5);
     const DevParam& P = d.params[d.meta[self] & META_PID_MASK];
     const float delta = P.deltaf;
     const float4 hi = d.uhi[self], lo = d.ulo[self];
-    const float2 nhi = make_float2(-hi.x, -hi.y), nlo = make_float2(-lo.x, -lo.y);
-    const float nhz = -hi.z, nlz = -lo.z;
+    const Own32 own(hi, lo);
     const float4 ci0 = d.cst32[3 * (long long)self], ci1 = d.cst32[3 * (long long)self + 1],
                  ci2 = d.cst32[3 * (long long)self + 2];
-    KSum2 bxy;
-    KSum1 bz;
-    Stream32<CLS, false> st(d, &tab, s, sbase, rows, lane, self);
+    const int* pn = d.nbr + sbase + lane;
+    const float4* pg = d.geo + sbase + lane;
+    const unsigned* pw = d.bits + (sbase >> 5);
+    KSum2 bxy, sxy;  // the sums of the segment and of the point
+    KSum1 bz, sz;
+    int nj0 = self, nj1 = self;
+    float4 ng0 = make_float4(0.f, 0.f, 0.f, 1.f), ng1 = ng0;
+    unsigned nw0 = 0u, nw1 = 0u;
+    auto load_pair = [&](int r) {
+      const bool two = r + 1 < rows;
+      nw0 = ld_stream(pw + r);
+      nw1 = two ? ld_stream(pw + r + 1) : 0u;
+      nj0 = ld_stream(pn + 32 * r);
+      ng0 = ld_stream(pg + 32 * r);
+      if (two) { nj1 = ld_stream(pn + 32 * r + 32); ng1 = ld_stream(pg + 32 * r + 32); }
+      else { nj1 = self; ng1 = make_float4(0.f, 0.f, 0.f, 1.f); }
+    };
+    if (rows > 0) load_pair(0);
     for (int r = 0; r < rows; r += 2) {
-      unsigned w0, w1;
-      bool a0, a1;
-      int j0, j1;
-      float4 g0, g1;
-      st.take(r, w0, w1, a0, a1, j0, j1, g0, g1);
+      const bool a0 = (nw0 >> lane) & 1u, a1 = (nw1 >> lane) & 1u;
+      const int j0 = a0 ? nj0 : self, j1 = a1 ? nj1 : self;
+      const float4 g0 = ng0, g1 = ng1;
       const float4 hj0 = __ldg(d.uhi + j0), lj0 = __ldg(d.ulo + j0);
       const float4 hj1 = __ldg(d.uhi + j1), lj1 = __ldg(d.ulo + j1);
       const float4* cj0 = d.cst32 + 3 * (long long)j0;
       const float4* cj1 = d.cst32 + 3 * (long long)j1;
       const float4 c00 = __ldg(cj0), c01 = __ldg(cj0 + 1), c02 = __ldg(cj0 + 2);
       const float4 c10 = __ldg(cj1), c11 = __ldg(cj1 + 1), c12 = __ldg(cj1 + 2);
-      if (r + 2 < rows) st.load(r + 2);
+      if (r + 2 < rows) load_pair(r + 2);
 #pragma unroll
       for (int u = 0; u < 2; u++) {
         const float4& g = u ? g1 : g0;
@@ -1125,35 +940,25 @@ __global__ void __launch_bounds__(256, PD_MINB_CQB) k_c_b32q(DevBody d, int kste
         const float4& c0 = u ? c10 : c00;
         const float4& c1 = u ? c11 : c01;
         const float4& c2 = u ? c12 : c02;
-        const float2 dxy = add2(add2(xy(hj), nhi), add2(xy(lj), nlo));
-        const float dz = (hj.z + nhz) + (lj.z + nlz);
-        // S = A_i + A_j (column-major: columns (S0 S1 S2), (S3 S4 S5), (S6 S7 S8)); beta_i + beta_j
-        const float2 S01 = add2(make_float2(ci0.x, ci0.y), make_float2(c0.x, c0.y));
-        const float2 S23 = add2(make_float2(ci0.z, ci0.w), make_float2(c0.z, c0.w));
-        const float2 S45 = add2(make_float2(ci1.x, ci1.y), make_float2(c1.x, c1.y));
-        const float2 S67 = add2(make_float2(ci1.z, ci1.w), make_float2(c1.z, c1.w));
-        const float2 S8b = add2(make_float2(ci2.x, ci2.y), make_float2(c2.x, c2.y));
-        // rows x, y: S01 xi_x + (S3, S4) xi_y + S67 xi_z + beta du
-        const float2 S34 = make_float2(S23.y, S45.x);
-        float2 txy = mul2(make_float2(S8b.y, S8b.y), dxy);
-        txy = add2(txy, mul2(S01, make_float2(g.x, g.x)));
-        txy = add2(txy, mul2(S34, make_float2(g.y, g.y)));
-        txy = add2(txy, mul2(S67, make_float2(g.z, g.z)));
-        const float tz = fmaf(S23.x, g.x, fmaf(S45.y, g.y, fmaf(S8b.x, g.z, S8b.y * dz)));
-        const float L = fabsf(g.w);
-        float f = omega_of_f(LIN ? KER_LINEAR : d.kernel, delta, L) * hj.w;
+        float2 dxy, txy;
+        float dz, num, tz;
+        bond_du(g, hj, lj, own, dxy, dz, num);
+        corr_pair(g, dxy, dz, ci0, ci1, make_float2(ci2.x, ci2.y), c0, c1, make_float2(c2.x, c2.y), txy, tz);
+        float f = (LIN ? bond_rl(g.w) : omega_of_f(d.kernel, delta, fabsf(g.w))) * hj.w;
         f = (u ? a1 : a0) ? f : 0.f;
         bxy.add(mul2(make_float2(f, f), txy));
         bz.add(f * tz);
       }
+      if ((r + 2) % SEG32 == 0 || r + 2 >= rows) {
+        join(sxy, bxy);
+        join(sz, bz);
+        bxy = KSum2();
+        bz = KSum1();
+      }
     }
     if (valid) {
-      const float2 v = bxy.value();
-      const float z = bz.value();
-      d.b32[3 * i] = v.x;
-      d.b32[3 * i + 1] = v.y;
-      d.b32[3 * i + 2] = z;
-      flag_nan32(d, kstep, v.x, v.y, z);
+      // the linear influence function is delta / L: delta leaves the sums
+      store_force(d, i, kstep, LIN ? P.delta : 1.0, sxy.value(), sz.value());
     }
   }
 }
@@ -1241,22 +1046,11 @@ static int launch_osb32(const DevBody& d, const LaunchCfg& c, int G, int grid, i
   return launches;
 }
 
-template <bool CLS>
-static void launch_c_a32q(const DevBody& d, const LaunchCfg& c, int grid, int kstep, cudaStream_t s) {
-  const bool lin = d.kernel == KER_LINEAR;
-  if (c.fullk) {
-    if (lin) k_c_a32q<CLS, true, true><<<grid, c.block, 0, s>>>(d, kstep);
-    else k_c_a32q<CLS, true, false><<<grid, c.block, 0, s>>>(d, kstep);
-  } else {
-    if (lin) k_c_a32q<CLS, false, true><<<grid, c.block, 0, s>>>(d, kstep);
-    else k_c_a32q<CLS, false, false><<<grid, c.block, 0, s>>>(d, kstep);
-  }
-}
-
-template <bool CLS>
-static void launch_c_b32q(const DevBody& d, const LaunchCfg& c, int grid, int kstep, cudaStream_t s) {
-  if (d.kernel == KER_LINEAR) k_c_b32q<CLS, true><<<grid, c.block, 0, s>>>(d, kstep);
-  else k_c_b32q<CLS, false><<<grid, c.block, 0, s>>>(d, kstep);
+// The tile kernels (pd_tile32.cu) run wherever the packed kernels' conditions hold and the body has
+// tiles, whatever the bond-stream variant: they were the fastest of all variants at every size
+// measured (pd_tile32.cu).
+static bool on_tiles(const DevBody& d, int phase) {
+  return packed_supported(d, phase) && tile32_supported(d, phase);
 }
 
 int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s) {
@@ -1264,8 +1058,14 @@ int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, c
   const int grid = grid_for32(d.nslices, c.block);
   const bool A = phase != 2, B = phase != 1;
   int launches = 0;
+  if (d.material == MAT_BB && !A) return 0;
+  if (phase == 0 && d.material != MAT_BB)
+    return launch_force32(d, c, kstep, 1, s) + launch_force32(d, c, kstep, 2, s);
+  if (on_tiles(d, A ? 1 : 2)) {
+    launch_tile32(d, c, kstep, A ? 1 : 2, s);
+    return 1;
+  }
   if (d.material == MAT_BB) {
-    if (!A) return 0;
     if (c.pipe == 5 && pk_supported(d, 1)) return launch_force32_pk(d, c, kstep, 1, s);
     LaunchCfg c4 = c;
     if (c.pipe == 5) c4.pipe = 4;   // the two-row kernel where the packed one does not apply
@@ -1290,9 +1090,15 @@ int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, c
     if (d.sc32) return launch_osb32<true>(d, c, G, grid, kstep, A, B, s);
     return launch_osb32<false>(d, c, G, grid, kstep, A, B, s);
   }
+  const bool lin = d.kernel == KER_LINEAR;
   if (A && c.pipe == 5 && cq_supported(d, 1)) {
-    if (d.ncls > 0) launch_c_a32q<true>(d, c, grid, kstep, s);
-    else launch_c_a32q<false>(d, c, grid, kstep, s);
+    if (c.fullk) {
+      if (lin) k_c_a32q<true, true><<<grid, c.block, 0, s>>>(d, kstep);
+      else k_c_a32q<true, false><<<grid, c.block, 0, s>>>(d, kstep);
+    } else {
+      if (lin) k_c_a32q<false, true><<<grid, c.block, 0, s>>>(d, kstep);
+      else k_c_a32q<false, false><<<grid, c.block, 0, s>>>(d, kstep);
+    }
     launches++;
   } else if (A) {
     if (d.kernel == KER_LINEAR) {
@@ -1307,8 +1113,8 @@ int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, c
   }
   const bool wan = d.zem == ZEM_WAN;
   if (B && c.pipe == 5 && cq_supported(d, 2)) {
-    if (d.ncls > 0) launch_c_b32q<true>(d, c, grid, kstep, s);
-    else launch_c_b32q<false>(d, c, grid, kstep, s);
+    if (lin) k_c_b32q<true><<<grid, c.block, 0, s>>>(d, kstep);
+    else k_c_b32q<false><<<grid, c.block, 0, s>>>(d, kstep);
     launches++;
   } else if (B) {
     if (wan) {

@@ -224,8 +224,9 @@ template <int CR, int NS>
 __global__ void __launch_bounds__(128, PD_TMA_MINB) k_osb_a32t(DevBody d, int kstep) {
   PD_TMA_PROLOGUE(CR, NS)
   for (long long s = warp0; s < d.nslices && !timed_out; s += nwarps) {
-    const long long i = s * 32 + lane;
-    const bool valid = i < d.n;
+    const long long place = s * 32 + lane;
+    const bool valid = place < d.n;
+    const long long i = valid ? point_at(d, place) : place;
     const long long sbase = d.soff[s];
     const int rows = (int)((d.soff[s + 1] - sbase) >> 5);
     const int cnt = valid ? (int)(d.off[i + 1] - d.off[i]) : 0;
@@ -295,8 +296,9 @@ template <int CR, int NS, bool MULTI>
 __global__ void __launch_bounds__(128, PD_TMA_MINB) k_osb_b32t(DevBody d, int kstep) {
   PD_TMA_PROLOGUE(CR, NS)
   for (long long s = warp0; s < d.nslices && !timed_out; s += nwarps) {
-    const long long i = s * 32 + lane;
-    const bool valid = i < d.n;
+    const long long place = s * 32 + lane;
+    const bool valid = place < d.n;
+    const long long i = valid ? point_at(d, place) : place;
     const long long sbase = d.soff[s];
     const int rows = (int)((d.soff[s + 1] - sbase) >> 5);
     const int cnt = valid ? (int)(d.off[i + 1] - d.off[i]) : 0;
@@ -376,8 +378,9 @@ template <int CR, int NS, bool MULTI>
 __global__ void __launch_bounds__(128, PD_TMA_MINB) k_bb32t(DevBody d, int kstep) {
   PD_TMA_PROLOGUE(CR, NS)
   for (long long s = warp0; s < d.nslices && !timed_out; s += nwarps) {
-    const long long i = s * 32 + lane;
-    const bool valid = i < d.n;
+    const long long place = s * 32 + lane;
+    const bool valid = place < d.n;
+    const long long i = valid ? point_at(d, place) : place;
     const long long sbase = d.soff[s];
     const int rows = (int)((d.soff[s + 1] - sbase) >> 5);
     const int cnt = valid ? (int)(d.off[i + 1] - d.off[i]) : 0;

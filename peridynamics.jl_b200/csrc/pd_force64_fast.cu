@@ -105,8 +105,9 @@ struct Place {
     part = (int)(w % W);
     gl = lane % G;
     const bool live = s < d.nslices;
-    i = s * (32 / G) + lane / G;
-    valid = live && i < d.n;
+    const long long q = s * (32 / G) + lane / G;
+    valid = live && q < d.n;
+    i = valid ? point_at(d, q) : q;
     self = valid ? (int)i : 0;
     const long long sbase = live ? d.soff[s] : 0;
     rows = live ? (int)((d.soff[s + 1] - sbase) >> 5) : 0;
@@ -117,8 +118,9 @@ struct Place {
   }
 };
 
-// the stream of rows r .. r + RU - 1 (past the last row: row r again, with no state bit set)
-template <int RU, bool ESC, bool OWNED>
+// the stream of rows r .. r + RU - 1 (past the last row: row r again, with no state bit set; with
+// one lane per point the rows of a slice are a multiple of four)
+template <int G, int RU, bool ESC, bool OWNED>
 struct Rows {
   int j[RU];
   double L[RU], sc[ESC ? RU : 1];
@@ -128,7 +130,7 @@ struct Rows {
   __device__ __forceinline__ void load(const P& p, int r) {
 #pragma unroll
     for (int u = 0; u < RU; u++) {
-      const bool in = u == 0 || r + u < p.rows;
+      const bool in = (G == 1 && RU <= 2) || u == 0 || r + u < p.rows;
       const int q = in ? r + u : r;
       w[u] = OWNED ? p.bits[q] : __ldg(p.bits + q);
       if (!in) w[u] = 0u;
@@ -253,14 +255,14 @@ __global__ void __launch_bounds__(256, MB_BB) k_bb64f(DevBody d, int kstep) {
   const DevParam& P = d.params[p.valid ? d.meta[p.self] & META_PID_MASK : 0];
   const double epsc = P.epsc, thr = fail_threshold(epsc), bci = P.bc;
   Totals<W, 3, false> T(p.part, p.lane);
-  Rows<RU, ESC, true> nx;
+  Rows<G, RU, ESC, true> nx;
   if (p.part * SEG < p.rows) nx.load(p, p.part * SEG);
   for (int r0 = 0; r0 < p.rows; r0 += W * SEG) {
     double seg[3] = {0.0, 0.0, 0.0};
     int nseg = 0;
     const int ra = r0 + p.part * SEG, rb = min(ra + SEG, p.rows);
     for (int r = ra; r < rb; r += RU) {
-      const Rows<RU, ESC, true> c = nx;
+      const Rows<G, RU, ESC, true> c = nx;
       bool a[RU];
       int j[RU];
 #pragma unroll
@@ -324,14 +326,14 @@ __global__ void __launch_bounds__(256, MB_OA) k_osb_a64f(DevBody d, int kstep) {
   const DevParam& P = d.params[p.valid ? d.meta[p.self] & META_PID_MASK : 0];
   const double epsc = P.epsc, thr = fail_threshold(epsc), delta = P.delta;
   Totals<W, 2, false> T(p.part, p.lane);
-  Rows<RU, ESC, true> nx;
+  Rows<G, RU, ESC, true> nx;
   if (p.part * SEG < p.rows) nx.load(p, p.part * SEG);
   for (int r0 = 0; r0 < p.rows; r0 += W * SEG) {
     double seg[2] = {0.0, 0.0};
     int nseg = 0;
     const int ra = r0 + p.part * SEG, rb = min(ra + SEG, p.rows);
     for (int r = ra; r < rb; r += RU) {
-      const Rows<RU, ESC, true> c = nx;
+      const Rows<G, RU, ESC, true> c = nx;
       bool a[RU];
       int j[RU];
 #pragma unroll
@@ -395,13 +397,13 @@ __global__ void __launch_bounds__(256, MB_OB) k_osb_b64f(DevBody d, int kstep) {
   const double2 ci = *reinterpret_cast<const double2*>(d.coef64 + p.self);
   const double delta = d.params[p.valid ? d.meta[p.self] & META_PID_MASK : 0].delta;
   Totals<W, 3, false> T(p.part, p.lane);
-  Rows<RU, ESC, false> nx;
+  Rows<G, RU, ESC, false> nx;
   if (p.part * SEG < p.rows) nx.load(p, p.part * SEG);
   for (int r0 = 0; r0 < p.rows; r0 += W * SEG) {
     double seg[3] = {0.0, 0.0, 0.0};
     const int ra = r0 + p.part * SEG, rb = min(ra + SEG, p.rows);
     for (int r = ra; r < rb; r += RU) {
-      const Rows<RU, ESC, false> c = nx;
+      const Rows<G, RU, ESC, false> c = nx;
       bool a[RU];
       int j[RU];
 #pragma unroll
@@ -463,7 +465,7 @@ __global__ void __launch_bounds__(256, MB_CA) k_c_a64f(DevBody d, int kstep) {
   const double f1 = 1.0 + epsc;
   const double sure = epsc > -0.5 ? f1 * f1 * (1.0 - 2e-14) : 0.0;
   Totals<W, 15, true> T(p.part, p.lane);
-  Rows<RU, false, true> nx;
+  Rows<G, RU, false, true> nx;
   if (p.part * SEG < p.rows) nx.load(p, p.part * SEG);
   for (int r0 = 0; r0 < p.rows; r0 += W * SEG) {
     double seg[15];
@@ -472,7 +474,7 @@ __global__ void __launch_bounds__(256, MB_CA) k_c_a64f(DevBody d, int kstep) {
     int nseg = 0;
     const int ra = r0 + p.part * SEG, rb = min(ra + SEG, p.rows);
     for (int r = ra; r < rb; r += RU) {
-      const Rows<RU, false, true> c = nx;
+      const Rows<G, RU, false, true> c = nx;
       bool a[RU];
       int j[RU];
 #pragma unroll
@@ -550,13 +552,13 @@ __global__ void __launch_bounds__(256, MB_CB) k_c_b64f(DevBody d, int kstep) {
 #pragma unroll
   for (int k = 0; k < 5; k++) Ai[k] = d.cst64[k * n + p.self];
   Totals<W, 3, false> T(p.part, p.lane);
-  Rows<RU, false, false> nx;
+  Rows<G, RU, false, false> nx;
   if (p.part * SEG < p.rows) nx.load(p, p.part * SEG);
   for (int r0 = 0; r0 < p.rows; r0 += W * SEG) {
     double seg[3] = {0.0, 0.0, 0.0};
     const int ra = r0 + p.part * SEG, rb = min(ra + SEG, p.rows);
     for (int r = ra; r < rb; r += RU) {
-      const Rows<RU, false, false> c = nx;
+      const Rows<G, RU, false, false> c = nx;
       const int nr = next_rows<W, RU>(r, ra, rb);
 #pragma unroll
       for (int u = 0; u < RU; u++) {

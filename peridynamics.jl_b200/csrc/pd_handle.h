@@ -70,7 +70,10 @@ struct pd_handle {
   // FP32 OSB / CMat: the stored weighted volumes / shape tensors are stale (bond states
   // changed outside the kernels)
   bool kfull = true;
-  bool cls_tried = false;  // bond classes were looked for in the current layout
+  bool tiles_tried = false;  // tiles and bond classes were looked for in the current layout
+  pd::PlaceGrid grid{};      // of the places of the one-lane layout
+  int* pt = nullptr;         // those places (kept while a lane-group layout is in use)
+  int* place = nullptr;
   bool damage_valid = false;
   bool has_bext_state = false;
   // boundary conditions (host side)

@@ -88,13 +88,35 @@ void launch_split_u(const DevBody& d, cudaStream_t s);
 // the split of rows[0 .. n) (halo rows that received a displacement)
 void launch_split_u_rows(const DevBody& d, const int* rows, long long n, cudaStream_t s);
 
+// places and tiles (pd_tiles.cu): the lattice of the places (its origin, the inverse spacing, the
+// axes in the order they are used), the places of the points, and the tiles of eight slices. The
+// arrays are the caller's to free; a body with a tile of more than TILE_MAX points has no tiles
+// (pt null)
+constexpr int TILE_MAX = 4095;  // 16-byte records that a 16-bit byte offset reaches
+struct PlaceGrid {
+  double lo[3], inv;
+  int axis[3];
+};
+struct TileArrays {
+  int* pt;
+  int* n;
+  uint2* lidx;
+  unsigned short* lown;
+  int cap;
+};
+cudaError_t build_places(const DevBody& d, const PlaceGrid& g, int** pt, int** place, cudaStream_t s);
+cudaError_t build_tiles(const DevBody& d, long long nslots, TileArrays* out, cudaStream_t s);
 // bond classes of an FP32 body with one lane per point (pd_classes.cu): *ncls = 0 when the bonds
 // fall into more than 256. The arrays are the caller's to free
-cudaError_t build_classes(const DevBody& d, long long nslots, unsigned** cls, float4** geo, int** dj,
-                          int* ncls, cudaStream_t s);
+constexpr int MAX_CLASSES = 256;
+cudaError_t build_classes(const DevBody& d, long long nslots, unsigned** cls, float4** geo, int* ncls,
+                          cudaStream_t s);
+// the tile kernels (pd_tile32.cu) of a phase (1: the first, 2: the second) of an FP32 body
+bool tile32_supported(const DevBody& d, int phase);
+void launch_tile32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s);
 
 // sliced bond layout and bond-array helpers (pd_layout.cu)
-cudaError_t build_slices(long long n, const long long* off, int G, long long** soff_out,
+cudaError_t build_slices(long long n, const long long* off, const int* pt, int G, long long** soff_out,
                          long long* nslices_out, long long* nslots_out, cudaStream_t s);
 void launch_scatter_i32(const DevBody& d, const int* src, int* dst, cudaStream_t s);
 void launch_relayout_i32(const DevBody& a, const DevBody& b, const int* src, int* dst, cudaStream_t s);

@@ -17,25 +17,30 @@ static inline int blocks_for(long long n, int t) {
   return (int)(b < 1 ? 1 : b);
 }
 
-// rows of 32 slots that slice s needs: ceil(max bond count of its points / G), times 32
-__global__ void k_slice_slots(long long n, const long long* off, int G, long long nslices,
-                              long long* slots) {
+// slots of slice s: rows of 32 for ceil(max bond count of its points / G) bonds a lane; with one
+// lane per point a multiple of four rows (1 % more at 122 bonds a point), so that kernels take
+// two and four rows at a time without a remainder
+__global__ void k_slice_slots(long long n, const long long* off, const int* pt, int G,
+                              long long nslices, long long* slots) {
   const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nslices) return;
   const int P = 32 / G;
   long long m = 0;
   for (int p = 0; p < P; p++) {
-    const long long i = s * P + p;
-    if (i < n) m = max(m, off[i + 1] - off[i]);
+    const long long q = s * P + p;
+    if (q >= n) continue;
+    const long long i = pt ? pt[q] : q;
+    m = max(m, off[i + 1] - off[i]);
   }
-  slots[s] = ((m + G - 1) / G) * 32;
+  const long long rows = (m + G - 1) / G;
+  slots[s] = 32 * (G == 1 ? (rows + 3) / 4 * 4 : rows);
 }
 
 __global__ void k_set_total(long long* soff, long long nslices, const long long* slots) {
   soff[nslices] = soff[nslices - 1] + slots[nslices - 1];
 }
 
-cudaError_t build_slices(long long n, const long long* off, int G, long long** soff_out,
+cudaError_t build_slices(long long n, const long long* off, const int* pt, int G, long long** soff_out,
                          long long* nslices_out, long long* nslots_out, cudaStream_t s) {
   const long long P = 32 / G;
   const long long ns = n > 0 ? (n + P - 1) / P : 1;
@@ -53,7 +58,7 @@ cudaError_t build_slices(long long n, const long long* off, int G, long long** s
     return cudaSuccess;
   }
   if (e == cudaSuccess) {
-    k_slice_slots<<<blocks_for(ns, 256), 256, 0, s>>>(n, off, G, ns, slots);
+    k_slice_slots<<<blocks_for(ns, 256), 256, 0, s>>>(n, off, pt, G, ns, slots);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, need, slots, soff, (int)ns, s);
@@ -166,8 +171,9 @@ __global__ void k_pack_bits(DevBody d, const unsigned char* bytes) {
   const int lane = threadIdx.x & 31, G = d.lg, P = 32 / G;
   const int sub = lane / G, gl = lane % G;
   const long long s = warp;
-  const long long i = s * P + sub;
-  const bool valid = i < d.n;
+  const long long q = s * P + sub;
+  const bool valid = q < d.n;
+  const long long i = valid ? point_at(d, q) : q;
   const long long sbase = d.soff[s];
   const int rows = (int)((d.soff[s + 1] - sbase) >> 5);
   const int cnt = valid ? (int)(d.off[i + 1] - d.off[i]) : 0;

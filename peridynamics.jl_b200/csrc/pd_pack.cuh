@@ -34,6 +34,13 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   return upk(d);
 }
 
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long d;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(pk(a)), "l"(pk(b)), "l"(pk(c)));
+  return upk(d);
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+
 // Kahan sum of pairs with the negated compensation n = -c: y = x + n, t = s + y,
 // n = (s - t) + y, s = t (the value is s + n)
 struct KSum2 {
