@@ -523,9 +523,10 @@ static int state_bytes(const DevBody& d, int phase) {
   return phase == 1 ? 0 : d.material == MAT_OSB ? 8 : 40;
 }
 
-// a tile and its classes fit the 227 KB of an SM
+// a tile, its classes and the segment sums of the warps that share a slice fit the 227 KB of a block
 bool tile32_supported(const DevBody& d, int phase) {
-  return d.tile_pt != nullptr && tile_bytes(d.tile_cap, state_bytes(d, phase), d.ncls) <= 227 * 1024;
+  return d.tile_pt != nullptr &&
+         tile_bytes(d.tile_cap, state_bytes(d, phase), d.ncls) + 8 * 1024 <= 227 * 1024;
 }
 
 // Warps per slice: the largest of 8, 4, 2, 1 that keeps the launch within the 24 warps per SM that

@@ -74,3 +74,18 @@ def test_result_does_not_depend_on_the_body_around(name):
         assert np.array_equal(many.field("bond_active", k), one.field("bond_active", 0))
     one.close()
     many.close()
+
+
+def test_tile_that_leaves_no_room_for_the_segment_sums():
+    """3,152 points a tile: the 72 bytes a point of CMat phase B fit a block's shared memory, but not
+    together with the sums of the warps that share a slice."""
+    body = box(MATERIALS["C"](), 23, 19, 21, 5.1, jitter=0.05)
+    ob = oracle_body(body)
+    u = deform(body._pos)
+    ob.pos[:] = body._pos + u
+    ob.force_density()
+    dev = pd.DeviceBody(body, precision="fp32")
+    dev.set_state(displacement=u)
+    dev.force()
+    assert np.abs(dev.field("b_int").T - ob.b_int).max() < 2e-5 * np.abs(ob.b_int).max()
+    dev.close()
