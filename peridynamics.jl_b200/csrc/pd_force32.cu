@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kste
     const DevParam& P = d.params[meta & META_PID_MASK];
     const float4 hi = d.uhi[self], lo = d.ulo[self];
     const Own32 own(hi, lo);
-    const CorrA cp(P, LIN);
+    const CorrA cp(d, P);
     const int* pn = d.nbr + sbase + lane;
     const float4* pg = d.geo + sbase + lane;
     unsigned* pw = d.bits + (sbase >> 5);
@@ -860,7 +860,7 @@ __global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kste
         bond_du(g, hj, u ? lj1 : lj0, own, dxy, dz, num);
         const float rL = bond_rl(g.w);
         const bool act = corr_stays(a, cp, g, rL, dxy, dz, num);
-        const float t = corr_weight<LIN>(d.kernel, cp, g, rL, hj.w);
+        const float t = corr_weight<LIN>(cp, g, rL, hj.w);
         S.add(act ? t : 0.f, g, dxy, dz);
         if (!FULLK && a && !act) S.drop(t, g);
         if (u) act1 = act; else act0 = act;
@@ -898,7 +898,7 @@ __global__ void __launch_bounds__(256, PD_MINB_CQB) k_c_b32q(DevBody d, int kste
     const long long sbase = d.soff[s];
     const int rows = (int)((d.soff[s + 1] - sbase) >> 5);
     const DevParam& P = d.params[d.meta[self] & META_PID_MASK];
-    const float delta = P.deltaf;
+    const Influence om(d, P);
     const float4 hi = d.uhi[self], lo = d.ulo[self];
     const Own32 own(hi, lo);
     const float4 ci0 = d.cst32[3 * (long long)self], ci1 = d.cst32[3 * (long long)self + 1],
@@ -944,7 +944,7 @@ __global__ void __launch_bounds__(256, PD_MINB_CQB) k_c_b32q(DevBody d, int kste
         float dz, num, tz;
         bond_du(g, hj, lj, own, dxy, dz, num);
         corr_pair(g, dxy, dz, ci0, ci1, make_float2(ci2.x, ci2.y), c0, c1, make_float2(c2.x, c2.y), txy, tz);
-        float f = (LIN ? bond_rl(g.w) : omega_of_f(d.kernel, delta, fabsf(g.w))) * hj.w;
+        float f = (LIN ? bond_rl(g.w) : om.at<LIN>(fabsf(g.w), 0.f)) * hj.w;
         f = (u ? a1 : a0) ? f : 0.f;
         bxy.add(mul2(make_float2(f, f), txy));
         bz.add(f * tz);

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256, PD_MINB_QB) k_osb_b32q(DevBody d, int kst
     const long long sbase = d.soff[s];
     const int rows = (int)((d.soff[s + 1] - sbase) >> 5);
     const DevParam& P = d.params[d.meta[self] & META_PID_MASK];
-    const float delta = P.deltaf;
+    const Influence om(d, P);
     const float4 hi = d.uhi[self], lo = d.ulo[self];
     const float2 ci = d.cc32[self];
     const Own32 own(hi, lo);
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(256, PD_MINB_QB) k_osb_b32q(DevBody d, int kst
         bond_pk(g, hj, u ? lj1 : lj0, own, B);
         const float rL = bond_rl(g.w);
         const float2 cs = add2(ci, u ? cj1 : cj0);
-        float f = osb_pair<LIN>(d.kernel, delta, B, rL, cs, hj.w);
+        float f = osb_pair<LIN>(om, B, rL, cs, hj.w);
         f = (u ? a1 : a0) ? f : 0.f;
         bxy.add(mul2(make_float2(f, f), B.exy));
         bz.add(f * B.ez);
@@ -139,7 +139,8 @@ __global__ void __launch_bounds__(256, PD_MINB_QA) k_osb_a32q(DevBody d, int kst
     const long long sbase = d.soff[s];
     const int rows = (int)((d.soff[s + 1] - sbase) >> 5);
     const DevParam& P = d.params[d.meta[self] & META_PID_MASK];
-    const float epsc = P.epscf, delta = P.deltaf;
+    const float epsc = P.epscf;
+    const Influence om(d, P);
     const float4 hi = d.uhi[self], lo = d.ulo[self];
     const Own32 own(hi, lo);
     const int* pn = d.nbr + sbase + lane;
@@ -182,12 +183,12 @@ __global__ void __launch_bounds__(256, PD_MINB_QA) k_osb_a32q(DevBody d, int kst
         bond_pk(g, hj, u ? lj1 : lj0, own, B);
         const float rL = bond_rl(g.w);
         const bool act = stays(a, B.e * rL, epsc, g.w);
-        const float th_b = act ? dil_term<LIN>(d.kernel, delta, B, rL, hj.w) : 0.f;
+        const float th_b = act ? dil_term<LIN>(om, B, rL, hj.w) : 0.f;
         if (FULLM) {
-          mt.add(make_float2(act ? vol_term<LIN>(d.kernel, delta, g, rL, hj.w) : 0.f, th_b));
+          mt.add(make_float2(act ? vol_term<LIN>(om, g, rL, hj.w) : 0.f, th_b));
         } else {
           th.add(th_b);
-          if (a && !act) dm += vol_term<LIN>(d.kernel, delta, g, rL, hj.w);
+          if (a && !act) dm += vol_term<LIN>(om, g, rL, hj.w);
         }
         if (u) act1 = act; else act0 = act;
       }

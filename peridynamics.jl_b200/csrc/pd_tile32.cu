@@ -16,11 +16,12 @@
 // are those of pd_force32_pk.cu: the same bits.
 //
 // Time of a step, lattices at a horizon of 3.015 spacings, packed kernels before and tiles (us, CUDA
-// graphs): OSB 1M points 1003 -> 661, 4.24M 4381 -> 2701, jittered 1M 1056 -> 920; BB 1M 501 -> 354;
-// CMat 1M 1351 -> 962. Against the one-row kernels of an untuned body: OSB 975 points 65 -> 15,
-// 27,347 105 -> 37, 64,000 185 -> 69; CMat 64,000 212 -> 87. Phase A now issues 74 % of its slots with
-// the L1 pipe at 77 %, phase B 65 % with 83 %: the neighbour and class records read from shared memory
-// (12 wavefronts a row in phase A) are what is left. With the full geometry stream DRAM is at 56 %.
+// graphs): OSB 1M points 1003 -> 633, 4.24M 4381 -> 2600, jittered 1M 1056 -> 955; BB 1M 501 -> 356;
+// CMat 320k 464 -> 314, 125k 232 -> 184. Against the one-row kernels of an untuned body: OSB 975 points
+// 65 -> 15, 27,347 105 -> 37, 64,000 185 -> 69; CMat 64,000 212 -> 87. OSB phase A issues 75 % of its
+// slots with the L1 pipe at 63 %: arithmetic and the neighbour and class records read from shared
+// memory (12 wavefronts a row) are what is left. With the full geometry stream DRAM is at 56 %, and
+// copying it ahead asynchronously (4 to 8 rows in shared memory) changed no time by more than 3 %.
 //
 // Below the size at which tiles fill the chip, W warps of a block share a slice and W blocks a tile:
 // the slice's rows are cut into segments of SEG32 rows that are summed from zero and joined in row
@@ -55,10 +56,13 @@ struct Pair32 {
   unsigned cls[2];
 };
 
-// OWNED: the kernel rewrites its state words, which are therefore loaded plainly
+// A warp walks four rows at a time, with the neighbour places and classes of the four after them in
+// registers. The state words: OWNED, the kernel rewrites them, so they are loaded plainly, two rows
+// ahead; else four rows ahead as well (CMat phase B, 320k points: 212 -> 169 us, OSB phase B, 1M points:
+// 342 -> 314; with two blocks per SM the wait for two rows' words was the largest stall. In the OWNED
+// kernels the four registers cost more than the wait: OSB phase A 298 -> 350).
 template <bool CLS, bool OWNED>
 struct TileStream {
-  const char* sm;
   const float* rl;      // CLS: 1 / L of the classes
   const float4* geo;    // CLS: their records
   const unsigned* pw;
@@ -67,40 +71,41 @@ struct TileStream {
   const float4* pg;
   int rows;
   unsigned mask;
-  uint2 nw, li, ln;     // states of the next row pair; neighbour places of these and of the next four rows
-  unsigned cw, cn;
-  float4 ng0, ng1;
+  uint2 nw;             // OWNED: states of the next row pair
+  uint4 wi, wn;         // else: states of these four rows and of the next
+  uint2 li, ln;         // neighbour places
+  unsigned cw, cn;      // classes
+  float4 ng0, ng1;      // without classes: geometry of the next row pair
 
-  __device__ __forceinline__ TileStream(const DevBody& d, const char* smem, const float4* geo_,
-                                        const float* rl_, long long sbase, int rows_, int lane)
-      : sm(smem), rl(rl_), geo(geo_), pw(d.bits + (sbase >> 5)), pl(d.lidx + (sbase >> 2) + lane),
-        rows(rows_), mask(1u << lane) {
+  __device__ __forceinline__ TileStream(const DevBody& d, const float4* geo_, const float* rl_,
+                                        long long sbase, int rows_, int lane)
+      : rl(rl_), geo(geo_), pw(d.bits + (sbase >> 5)), pl(d.lidx + (sbase >> 2) + lane), rows(rows_),
+        mask(1u << lane) {
     if constexpr (CLS) pc = d.cls + (sbase >> 2) + lane;
     else pg = d.geo + sbase + lane;
   }
 
-  // the four rows from r on are the first that the warp walks
+  // the four rows from r on are the first that the warp walks, those from `after` the second
   __device__ __forceinline__ void start(int r, int after) {
     if (r >= rows) return;
-    ln = ld_stream(pl + 8 * r);
-    if constexpr (CLS) cn = ld_stream(pc + 8 * r);
+    fetch(r);
     load<0>(r, after);
   }
-
+  __device__ __forceinline__ void fetch(int r) {
+    if constexpr (!OWNED) wn = ld_stream(reinterpret_cast<const uint4*>(pw + r));
+    ln = ld_stream(pl + 8 * r);
+    if constexpr (CLS) cn = ld_stream(pc + 8 * r);
+  }
   // the records of rows r and r + 1; H: the second pair of its four rows; else the four rows that the
   // warp walks after them start at `after`
   template <int H>
   __device__ __forceinline__ void load(int r, int after) {
-    const uint2* q = reinterpret_cast<const uint2*>(pw + r);
-    if constexpr (OWNED) nw = *q;
-    else nw = ld_stream(q);
+    if constexpr (OWNED) nw = *reinterpret_cast<const uint2*>(pw + r);
     if constexpr (H == 0) {
+      if constexpr (!OWNED) wi = wn;
       li = ln;
       if constexpr (CLS) cw = cn;
-      if (after < rows) {
-        ln = ld_stream(pl + 8 * after);
-        if constexpr (CLS) cn = ld_stream(pc + 8 * after);
-      }
+      if (after < rows) fetch(after);
     }
     if constexpr (!CLS) {
       ng0 = ld_stream(pg + 32 * r);
@@ -111,10 +116,10 @@ struct TileStream {
   template <int H>
   __device__ __forceinline__ void take(Pair32& p) const {
     const unsigned v = H ? li.y : li.x;
-    p.w[0] = nw.x;
-    p.w[1] = nw.y;
-    p.a[0] = (nw.x & mask) != 0u;
-    p.a[1] = (nw.y & mask) != 0u;
+    p.w[0] = OWNED ? nw.x : H ? wi.z : wi.x;
+    p.w[1] = OWNED ? nw.y : H ? wi.w : wi.y;
+    p.a[0] = (p.w[0] & mask) != 0u;
+    p.a[1] = (p.w[1] & mask) != 0u;
     p.key[0] = v & 0xffffu;
     p.key[1] = v >> 16;
     if constexpr (CLS) {
@@ -315,7 +320,7 @@ __global__ void __launch_bounds__(256, MT_BB) k_bb32s(DevBody d, int kstep) {
   const DevParam& P = d.params[t.valid ? d.meta[t.i] & META_PID_MASK : 0];
   const float epsc = P.epscf;
   const Own32 own(t.hi(t.own), t.lo(t.own));
-  TileStream<CLS, true> st(d, t.sm, t.geo, t.rl, t.sbase, t.rows, t.lane);
+  TileStream<CLS, true> st(d, t.geo, t.rl, t.sbase, t.rows, t.lane);
   const ForceSum S = walk_rows<W, ForceSum>(st, t.rows, t.part, t.lane, [&](const Pair32& p, int r, ForceSum& s) {
     bool act[2];
 #pragma unroll
@@ -346,9 +351,10 @@ __global__ void __launch_bounds__(256, MT_A) k_osb_a32s(DevBody d, int kstep) {
   Tile<CLS, 0, W> t;
   if (!t.begin(d, tile_smem)) return;
   const DevParam& P = d.params[t.valid ? d.meta[t.i] & META_PID_MASK : 0];
-  const float epsc = P.epscf, delta = P.deltaf;
+  const float epsc = P.epscf;
+  const Influence om(d, P);
   const Own32 own(t.hi(t.own), t.lo(t.own));
-  TileStream<CLS, true> st(d, t.sm, t.geo, t.rl, t.sbase, t.rows, t.lane);
+  TileStream<CLS, true> st(d, t.geo, t.rl, t.sbase, t.rows, t.lane);
   using Sum = DilSum<FULLM>;
   const Sum S = walk_rows<W, Sum>(st, t.rows, t.part, t.lane, [&](const Pair32& p, int r, Sum& s) {
     bool act[2];
@@ -359,9 +365,9 @@ __global__ void __launch_bounds__(256, MT_A) k_osb_a32s(DevBody d, int kstep) {
       bond_pk(p.g[u], hj, t.lo(p.key[u]), own, B);
       const float rL = st.rL(p, u);
       act[u] = stays(p.a[u], B.e * rL, epsc, p.g[u].w);
-      const float th_b = act[u] ? dil_term<LIN>(d.kernel, delta, B, rL, hj.w) : 0.f;
+      const float th_b = act[u] ? dil_term<LIN>(om, B, rL, hj.w) : 0.f;
       if constexpr (FULLM) {
-        s.mt.add(make_float2(act[u] ? vol_term<LIN>(d.kernel, delta, p.g[u], rL, hj.w) : 0.f, th_b));
+        s.mt.add(make_float2(act[u] ? vol_term<LIN>(om, p.g[u], rL, hj.w) : 0.f, th_b));
         s.na += (int)act[u];
       } else {
         s.th.add(th_b);
@@ -373,7 +379,7 @@ __global__ void __launch_bounds__(256, MT_A) k_osb_a32s(DevBody d, int kstep) {
 #pragma unroll
         for (int u = 0; u < 2; u++)
           if (p.a[u] && !act[u]) {
-            s.dm += vol_term<LIN>(d.kernel, delta, p.g[u], st.rL(p, u), t.hi(p.key[u]).w);
+            s.dm += vol_term<LIN>(om, p.g[u], st.rL(p, u), t.hi(p.key[u]).w);
             s.na++;
           }
       }
@@ -405,17 +411,17 @@ __global__ void __launch_bounds__(256, MT_B) k_osb_b32s(DevBody d, int kstep) {
   Tile<CLS, 8, W> t;
   if (!t.begin(d, tile_smem)) return;
   const DevParam& P = d.params[t.valid ? d.meta[t.i] & META_PID_MASK : 0];
-  const float delta = P.deltaf;
+  const Influence om(d, P);
   const Own32 own(t.hi(t.own), t.lo(t.own));
   const float2 ci = t.s8(t.own);
-  TileStream<CLS, false> st(d, t.sm, t.geo, t.rl, t.sbase, t.rows, t.lane);
+  TileStream<CLS, false> st(d, t.geo, t.rl, t.sbase, t.rows, t.lane);
   const ForceSum S = walk_rows<W, ForceSum>(st, t.rows, t.part, t.lane, [&](const Pair32& p, int r, ForceSum& s) {
 #pragma unroll
     for (int u = 0; u < 2; u++) {
       const float4 hj = t.hi(p.key[u]);
       BondP B;
       bond_pk(p.g[u], hj, t.lo(p.key[u]), own, B);
-      const float f = osb_pair<LIN>(d.kernel, delta, B, st.rL(p, u), add2(ci, t.s8(p.key[u])), hj.w);
+      const float f = osb_pair<LIN>(om, B, st.rL(p, u), add2(ci, t.s8(p.key[u])), hj.w);
       s.add(p.a[u] ? f : 0.f, B.exy, B.ez);
     }
   });
@@ -437,10 +443,10 @@ __global__ void __launch_bounds__(256, MT_CA) k_c_a32s(DevBody d, int kstep) {
   if (!t.begin(d, tile_smem)) return;
   const unsigned meta = t.valid ? d.meta[t.i] : 0u;
   const DevParam& P = d.params[meta & META_PID_MASK];
-  const CorrA cp(P, LIN);
+  const CorrA cp(d, P);
   const Own32 own(t.hi(t.own), t.lo(t.own));
   CorrAcc<FULLK> S;
-  TileStream<CLS, true> st(d, t.sm, t.geo, t.rl, t.sbase, t.rows, t.lane);
+  TileStream<CLS, true> st(d, t.geo, t.rl, t.sbase, t.rows, t.lane);
   auto pair = [&](const Pair32& p, int r) {
     bool act[2];
 #pragma unroll
@@ -451,7 +457,7 @@ __global__ void __launch_bounds__(256, MT_CA) k_c_a32s(DevBody d, int kstep) {
       bond_du(p.g[u], hj, t.lo(p.key[u]), own, dxy, dz, num);
       const float rL = st.rL(p, u);
       act[u] = corr_stays(p.a[u], cp, p.g[u], rL, dxy, dz, num);
-      const float w = corr_weight<LIN>(d.kernel, cp, p.g[u], rL, hj.w);
+      const float w = corr_weight<LIN>(cp, p.g[u], rL, hj.w);
       S.add(act[u] ? w : 0.f, p.g[u], dxy, dz);
       if (FULLK) S.na += (int)act[u];
     }
@@ -461,7 +467,7 @@ __global__ void __launch_bounds__(256, MT_CA) k_c_a32s(DevBody d, int kstep) {
 #pragma unroll
         for (int u = 0; u < 2; u++)
           if (p.a[u] && !act[u]) {
-            S.drop(corr_weight<LIN>(d.kernel, cp, p.g[u], st.rL(p, u), t.hi(p.key[u]).w), p.g[u]);
+            S.drop(corr_weight<LIN>(cp, p.g[u], st.rL(p, u), t.hi(p.key[u]).w), p.g[u]);
             S.na++;
           }
       }
@@ -498,11 +504,11 @@ __global__ void __launch_bounds__(256, MT_CB) k_c_b32s(DevBody d, int kstep) {
   Tile<CLS, 40, W> t;
   if (!t.begin(d, tile_smem)) return;
   const DevParam& P = d.params[t.valid ? d.meta[t.i] & META_PID_MASK : 0];
-  const float delta = P.deltaf;
+  const Influence om(d, P);
   const Own32 own(t.hi(t.own), t.lo(t.own));
   const float4 ia = t.sa(t.own), ib = t.sb(t.own);
   const float2 ic = t.sc(t.own);
-  TileStream<CLS, false> st(d, t.sm, t.geo, t.rl, t.sbase, t.rows, t.lane);
+  TileStream<CLS, false> st(d, t.geo, t.rl, t.sbase, t.rows, t.lane);
   const ForceSum S = walk_rows<W, ForceSum>(st, t.rows, t.part, t.lane, [&](const Pair32& p, int r, ForceSum& s) {
 #pragma unroll
     for (int u = 0; u < 2; u++) {
@@ -511,7 +517,7 @@ __global__ void __launch_bounds__(256, MT_CB) k_c_b32s(DevBody d, int kstep) {
       float dz, num, tz;
       bond_du(p.g[u], hj, t.lo(p.key[u]), own, dxy, dz, num);
       corr_pair(p.g[u], dxy, dz, ia, ib, ic, t.sa(p.key[u]), t.sb(p.key[u]), t.sc(p.key[u]), txy, tz);
-      const float f = (LIN ? st.rL(p, u) : omega_of_f(d.kernel, delta, fabsf(p.g[u].w))) * hj.w;
+      const float f = (LIN ? st.rL(p, u) : om.at<LIN>(fabsf(p.g[u].w), 0.f)) * hj.w;
       s.add(p.a[u] ? f : 0.f, txy, tz);
     }
   });
@@ -525,8 +531,7 @@ static int state_bytes(const DevBody& d, int phase) {
 
 // a tile, its classes and the segment sums of the warps that share a slice fit the 227 KB of a block
 bool tile32_supported(const DevBody& d, int phase) {
-  return d.tile_pt != nullptr &&
-         tile_bytes(d.tile_cap, state_bytes(d, phase), d.ncls) + 8 * 1024 <= 227 * 1024;
+  return d.tile_pt != nullptr && tile_bytes(d.tile_cap, state_bytes(d, phase), d.ncls) + 8 * 1024 <= 227 * 1024;
 }
 
 // Warps per slice: the largest of 8, 4, 2, 1 that keeps the launch within the 24 warps per SM that
