@@ -141,11 +141,11 @@ static pd_status check_symmetry(pd_handle* h) {
   return PD_OK;
 }
 
-// FP32 bodies with one lane per point gather from tiles in shared memory and, on a regular lattice,
-// read a bond's geometry as one byte. Both are made once per layout; a body without tiles or
+// Bodies with one lane per point gather from tiles in shared memory (FP64: BB and OSB) and, in FP32
+// on a regular lattice, read a bond's geometry as one byte. Both are made once per layout; a body without tiles or
 // classes, or without the memory for them, runs the kernels that its bond-stream variant names.
 static pd_status ensure_tiles(pd_handle* h) {
-  if (h->tiles_tried || h->precision == PD_PREC_FP64 || !packed_supported(h->d, 1))
+  if (h->tiles_tried || h->d.lg != 1 || h->d.pt == nullptr || h->multi)
     return PD_OK;
   h->tiles_tried = true;
   TileArrays t;
@@ -160,6 +160,7 @@ static pd_status ensure_tiles(pd_handle* h) {
   h->d.lown = t.lown;
   h->d.tile_cap = t.cap;
   h->version++;
+  if (h->precision == PD_PREC_FP64) return PD_OK;
   unsigned* cls = nullptr;
   float4* geo = nullptr;
   int ncls = 0;
@@ -194,7 +195,7 @@ static pd_status finish_create(pd_handle* h, int* dnbr_csr, const double* dL, co
   }
   long long* soff = nullptr;
   long long ns = 0, nslots = 0;
-  if (h->precision != PD_PREC_FP64) {
+  if (h->precision != PD_PREC_FP64 || h->material != PD_MAT_CMAT) {
     PD_CUDA(build_places(h->d, h->grid, &h->pt, &h->place, h->stream));
     h->allocs.push_back(h->pt);
     h->allocs.push_back(h->place);

@@ -5,8 +5,8 @@
 //   off      int64[n+1]   n_neighbors of point i is off[i+1] - off[i] (the reference's CSR
 //                         order: bond k of point i is bond off[i] + k of the reference)
 //   Bond arrays are stored in a sliced layout with G lanes per point ("SELL"): the points
-//   are cut into slices of P = 32 / G points (consecutive ones; FP32 with one lane per point: compact
-//   parts of the body, pd_tiles.cu); slice s owns rows
+//   are cut into slices of P = 32 / G points (consecutive ones; with one lane per point compact parts
+//   of the body, pd_tiles.cu); slice s owns rows
 //   [soff[s] / 32, soff[s+1] / 32) of 32 bond slots; bond k of the point p of the slice sits
 //   in row k / G at lane p * G + k % G. A warp walks one slice row by row, so every
 //   bond-array load of a warp is one contiguous 128-byte (int32) or 512-byte (float4)
@@ -91,7 +91,7 @@ struct DevBody {
   const int* rev;    // revk
   const double* len64;
   const float4* geo;
-  // one lane per point, FP32: the points in the order of their places in the slices (place q is
+  // one lane per point (FP64: BB and OSB): the points in the order of their places in the slices (place q is
   // lane q % 32 of slice q / 32) and the inverse; null where the places are the points
   const int* pt;
   const int* place;

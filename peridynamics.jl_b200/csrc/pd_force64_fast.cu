@@ -29,6 +29,7 @@
 // CUDA graphs): 3,200 points BB 55.6 -> 10.9, OSB 129 -> 17.5, CMat 237 -> 24; 27,347 points BB 70
 // -> 23, OSB 163 -> 42, CMat 301 -> 77; 125,000 points BB 153 -> 101, OSB 401 -> 190, CMat 920 ->
 // 281; 397,243 points BB 376 -> 268, OSB 1049 -> 498.
+#include "pd_bond64.cuh"
 #include "pd_common.cuh"
 #include "pd_launch.h"
 #include "pd_math64.cuh"
@@ -45,24 +46,7 @@ namespace {
 // (one row of stream 158, 3 blocks 240).
 constexpr int MB_BB = 3, MB_OA = 3, MB_OB = 3, MB_CA = 2, MB_CB = 2;
 constexpr int RU_BB = 2, RU_OA = 2, RU_OB = 2, RU_CA = 2, RU_CB = 2;
-constexpr int SEG = 16;  // rows of a segment (even)
-
-// 1 / sqrt(x) from the hardware's approximation y by one step of third order: with
-// e = 1 - x y^2, 1 / sqrt(x) = y (1 - e)^(-1/2) = y (1 + e / 2 + 3 e^2 / 8 + O(e^3))
-__device__ __forceinline__ double rsqrt3(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
-// 1 / x likewise: with e = 1 - x y, 1 / x = y / (1 - e) = y (1 + e + e^2 + O(e^3))
-__device__ __forceinline__ double rcp3(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
+constexpr int SEG = SEG64;
 
 // a point record {x, y, z, V} in one 256-bit load: the 32 lanes of a warp read 32 neighbouring
 // records, and two 128-bit loads would each touch every one of their sectors
@@ -71,12 +55,6 @@ __device__ __forceinline__ double4 ld_point(const double4* p) {
   asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
       : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
   return v;
-}
-
-// sqrt(x), with h an approximation of 1 / sqrt(x) to about an ulp
-__device__ __forceinline__ double sqrt_of(double x, double h) {
-  const double l = x * h;
-  return fma(fma(-l, l, x), 0.5 * h, l);
 }
 
 // An error of an earlier kernel ends the run. With several warps per slice the decision is the
@@ -221,25 +199,6 @@ __device__ __forceinline__ int next_rows(int r, int ra, int rb) {
   return r + RU < rb ? r + RU : ra + W * SEG;
 }
 
-// eps = (l - L) / L > eps_c: the division only where l - L is not clearly below eps_c L.
-// thr = eps_c less a margin far above the rounding of either side, -inf for eps_c <= 0
-__device__ __forceinline__ double fail_threshold(double epsc) {
-  return epsc > 0 ? epsc * (1.0 - 1e-14) : (epsc <= 0 ? -INFINITY : epsc);
-}
-__device__ __forceinline__ bool fails64(double l2, double e, double Ls, double L, double thr,
-                                        double epsc) {
-  if (!(Ls > 0) || e < thr * L) return false;
-  return (sqrt(l2) - L) / L > epsc;
-}
-
-__device__ __forceinline__ void nan_flag(const DevBody& d, int kstep, double x, double y, double z) {
-  if (isnan(x) || isnan(y) || isnan(z)) {
-    const long long step = d.ctrl->base + kstep;
-    if (atomicExch(&d.ctrl->err, 1) == 0) d.ctrl->err_step = step;
-    else atomicMin(&d.ctrl->err_step, step);
-  }
-}
-
 }  // namespace
 
 // -------------------------------------------------------------------------------------------
@@ -278,16 +237,13 @@ __global__ void __launch_bounds__(256, MB_BB) k_bb64f(DevBody d, int kstep) {
       bool act[RU];
 #pragma unroll
       for (int u = 0; u < RU; u++) {
-        const double L = fabs(c.L[u]);
         const double dx = x[u].x - xi.x, dy = x[u].y - xi.y, dz = x[u].z - xi.z;
-        const double l2 = (dx * dx + dy * dy) + dz * dz;
-        const double g = rsqrt3(l2 * (L * L));
-        const double e = sqrt_of(l2, g * L) - L;
-        act[u] = a[u] && !fails64(l2, e, c.L[u], L, thr, epsc);
+        const Bond64 b(dx, dy, dz, c.L[u]);
+        act[u] = a[u] && !fails64(b.l2, b.e, c.L[u], b.L, thr, epsc);
         double bc = bci;
         if (MULTI) bc = 0.5 * (bci + d.params[d.meta[j[u]] & META_PID_MASK].bc);
         if (ESC) bc *= c.sc[u];
-        const double sc = act[u] ? (bc * x[u].w) * (e * g) : 0.0;
+        const double sc = act[u] ? (bc * x[u].w) * (b.e * b.g) : 0.0;
         seg[0] = fma(sc, dx, seg[0]);
         seg[1] = fma(sc, dy, seg[1]);
         seg[2] = fma(sc, dz, seg[2]);
@@ -324,7 +280,7 @@ __global__ void __launch_bounds__(256, MB_OA) k_osb_a64f(DevBody d, int kstep) {
   const Place<G, W> p(d, ESC);
   const double4 xi = ld4_64(d.cur + p.self);
   const DevParam& P = d.params[p.valid ? d.meta[p.self] & META_PID_MASK : 0];
-  const double epsc = P.epsc, thr = fail_threshold(epsc), delta = P.delta;
+  const double epsc = P.epsc, thr = fail_threshold(epsc), delta = P.delta, rdelta = 1.0 / delta;
   Totals<W, 2, false> T(p.part, p.lane);
   Rows<G, RU, ESC, true> nx;
   if (p.part * SEG < p.rows) nx.load(p, p.part * SEG);
@@ -355,7 +311,7 @@ __global__ void __launch_bounds__(256, MB_OA) k_osb_a64f(DevBody d, int kstep) {
         const double e = sqrt_of(l2, rsqrt3(l2)) - L;
         act[u] = a[u] && !fails64(l2, e, c.L[u], L, thr, epsc);
         double t = ESC ? c.sc[u] * x[u].w : x[u].w;
-        if (!LIN) t *= omega_of(d.kernel, delta, L) * L;
+        if (!LIN) t *= omega64(d.kernel, delta, rdelta, L) * L;
         seg[0] = fma(act[u] ? t : 0.0, L, seg[0]);
         seg[1] += act[u] ? t * e : 0.0;
       }
@@ -395,7 +351,7 @@ __global__ void __launch_bounds__(256, MB_OB) k_osb_b64f(DevBody d, int kstep) {
   const Place<G, W> p(d, ESC);
   const double4 xi = ld4_64(d.cur + p.self);
   const double2 ci = *reinterpret_cast<const double2*>(d.coef64 + p.self);
-  const double delta = d.params[p.valid ? d.meta[p.self] & META_PID_MASK : 0].delta;
+  const double delta = d.params[p.valid ? d.meta[p.self] & META_PID_MASK : 0].delta, rdelta = 1.0 / delta;
   Totals<W, 3, false> T(p.part, p.lane);
   Rows<G, RU, ESC, false> nx;
   if (p.part * SEG < p.rows) nx.load(p, p.part * SEG);
@@ -421,16 +377,13 @@ __global__ void __launch_bounds__(256, MB_OB) k_osb_b64f(DevBody d, int kstep) {
       if (nr < p.rows) nx.load(p, nr);
 #pragma unroll
       for (int u = 0; u < RU; u++) {
-        const double L = fabs(c.L[u]);
         const double dx = x[u].x - xi.x, dy = x[u].y - xi.y, dz = x[u].z - xi.z;
-        const double l2 = (dx * dx + dy * dy) + dz * dz;
-        // g = 1 / (l L): omega / l = delta g (linear), omega L g otherwise
-        const double g = rsqrt3(l2 * (L * L));
-        const double e = sqrt_of(l2, g * L) - L;
-        const double t = fma(ci.y + cj[u].y, L, (ci.x + cj[u].x) * e);
-        double om = LIN ? delta : omega_of(d.kernel, delta, L) * L;
+        const Bond64 b(dx, dy, dz, c.L[u]);
+        const double t = fma(ci.y + cj[u].y, b.L, (ci.x + cj[u].x) * b.e);
+        // omega / l = delta g (linear), omega L g otherwise
+        double om = LIN ? delta : omega64(d.kernel, delta, rdelta, b.L) * b.L;
         if (ESC) om *= c.sc[u];
-        const double sc = a[u] ? (om * x[u].w) * (t * g) : 0.0;
+        const double sc = a[u] ? (om * x[u].w) * (t * b.g) : 0.0;
         seg[0] = fma(sc, dx, seg[0]);
         seg[1] = fma(sc, dy, seg[1]);
         seg[2] = fma(sc, dz, seg[2]);
@@ -461,7 +414,7 @@ __global__ void __launch_bounds__(256, MB_CA) k_c_a64f(DevBody d, int kstep) {
   const double4 xi = ld4_64(d.cur + p.self), Xi = ld4_64(d.X0 + p.self);
   const unsigned meta = p.valid ? d.meta[p.self] : 0u;
   const DevParam& P = d.params[meta & META_PID_MASK];
-  const double epsc = P.epsc, delta = P.delta;
+  const double epsc = P.epsc, delta = P.delta, rdelta = 1.0 / delta;
   const double f1 = 1.0 + epsc;
   const double sure = epsc > -0.5 ? f1 * f1 * (1.0 - 2e-14) : 0.0;
   Totals<W, 15, true> T(p.part, p.lane);
@@ -499,7 +452,7 @@ __global__ void __launch_bounds__(256, MB_CA) k_c_a64f(DevBody d, int kstep) {
         const double l2 = (dx * dx + dy * dy) + dz * dz;
         act[u] = a[u];
         if (a[u] && c.L[u] > 0 && !(l2 < sure * (L * L))) act[u] = !((sqrt(l2) - L) / L > epsc);
-        const double om = LIN ? delta * rcp3(L) : omega_of(d.kernel, delta, L);
+        const double om = LIN ? delta * rcp3(L) : omega64(d.kernel, delta, rdelta, L);
         const double t = act[u] ? om * x[u].w : 0.0;
         const double tx = t * DX, ty = t * DY, tz = t * DZ;
         seg[0] = fma(tx, DX, seg[0]); seg[1] = fma(ty, DY, seg[1]); seg[2] = fma(tz, DZ, seg[2]);
@@ -546,7 +499,7 @@ __global__ void __launch_bounds__(256, MB_CB) k_c_b64f(DevBody d, int kstep) {
   constexpr int RU = RU_CB;
   const Place<G, W> p(d, false);
   const double4 xi = ld4_64(d.cur + p.self), Xi = ld4_64(d.X0 + p.self);
-  const double delta = d.params[p.valid ? d.meta[p.self] & META_PID_MASK : 0].delta;
+  const double delta = d.params[p.valid ? d.meta[p.self] & META_PID_MASK : 0].delta, rdelta = 1.0 / delta;
   const long long n = d.n;
   double2 Ai[5];
 #pragma unroll
@@ -573,7 +526,7 @@ __global__ void __launch_bounds__(256, MB_CB) k_c_b64f(DevBody d, int kstep) {
         const double DX = X.x - Xi.x, DY = X.y - Xi.y, DZ = X.z - Xi.z;
         const double b = Ai[4].y + Aj[4].y;
         const double ux = (x.x - xi.x) - DX, uy = (x.y - xi.y) - DY, uz = (x.z - xi.z) - DZ;
-        const double om = LIN ? delta * rcp3(L) : omega_of(d.kernel, delta, L);
+        const double om = LIN ? delta * rcp3(L) : omega64(d.kernel, delta, rdelta, L);
         const double f = a ? om * x.w : 0.0;
         const double t0 = fma(Ai[0].x + Aj[0].x, DX, fma(Ai[1].y + Aj[1].y, DY, fma(Ai[3].x + Aj[3].x, DZ, b * ux)));
         const double t1 = fma(Ai[0].y + Aj[0].y, DX, fma(Ai[2].x + Aj[2].x, DY, fma(Ai[3].y + Aj[3].y, DZ, b * uy)));
@@ -682,6 +635,10 @@ static void launch_c64f(const DevBody& d, const Shape& q, int W, int kstep, int 
 }
 
 void launch_force64_fast(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s) {
+  if (tile64_supported(d, phase)) {
+    launch_tile64(d, kstep, phase, s);
+    return;
+  }
   const int W = warps_per_slice(d);
   const Shape q = shape_for(d, c, W);
   const bool lin = d.kernel == KER_LINEAR, esc = d.sc64 != nullptr;

@@ -66,6 +66,9 @@ int launch_force64(const DevBody& d, const LaunchCfg& c, int kstep, int phase, c
 // fast64_supported
 bool fast64_supported(const DevBody& d);
 void launch_force64_fast(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s);
+// the tile kernels (pd_tile64.cu) of BB and OSB
+bool tile64_supported(const DevBody& d, int phase);
+void launch_tile64(const DevBody& d, int kstep, int phase, cudaStream_t s);
 // the phase-B state of rows[0 .. n) (halo rows that received F and P K^-1)
 void launch_c_state_rows(const DevBody& d, const int* rows, long long n, cudaStream_t s);
 int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s);
