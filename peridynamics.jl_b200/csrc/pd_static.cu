@@ -6,14 +6,13 @@
 // a time loop that must not stall on the allocator, or an application that hands the library
 // memory it carved out of a fixed arena. For them pd_osb_force_static takes every input and
 // output as a device pointer owned by the caller and keeps its one piece of scratch state --
-// the weighted volume, dilatation and the two force coefficients of every point, which the
-// gather phase reads for the neighbours -- in the file-scope device array below. The array
+// the two force coefficients, the volume and the place of the bond list of every point, which the
+// gather phase reads for the neighbours in one 32-byte record -- in the file-scope device array below. The array
 // is part of the library image: every GPU that loads the library holds it until the process
 // exits, which is why it is kept to PD_STATIC_MAX_POINTS points (8 MiB).
 //
-// The arithmetic is the FP64 serial-order evaluation of pd_force64.cu (one thread per point,
-// the reference's order of operations and of the scattered terms), on the reference's CSR
-// bond arrays instead of the sliced layout.
+// The arithmetic is that of the FP64 kernels off the serial order (pd_bond64.cuh), on the reference's
+// CSR bond arrays instead of the sliced layout.
 #include <cuda.h>
 
 #include <mutex>
@@ -21,13 +20,18 @@
 #include <vector>
 
 #include "pdcuda.h"
+#include "pd_bond64.cuh"
 #include "pd_common.cuh"
 
 namespace pd {
 
 constexpr long long PD_STATIC_MAX_POINTS = 1LL << 18;
 
-// {c1, c2, wvol, dil} per point, shared by every call of pd_osb_force_static on this device
+// What bounds it: the gathers of the neighbours' positions, which reach L1 as three 8-byte loads of
+// records 24 bytes apart, and (phase B) the search for the reverse bond, which bounds jittered bodies.
+// us a call, one thread a point before / now: 1,380 points 481 / 42, 30,659 655 / 150, 147,420 1296 / 730.
+
+// {c1, c2, volume, place of the bond list} per point, shared by every call of pd_osb_force_static on this device
 static __device__ __align__(256) double4 g_osb_state[PD_STATIC_MAX_POINTS];
 
 struct StaticArgs {
@@ -47,6 +51,13 @@ struct StaticArgs {
   double4* state;     // g_osb_state, through the address looked up on the host
 };
 
+// the end of a point's bond list (below 2^44) and its size (a point has at most 2^18 neighbours)
+__device__ __forceinline__ double pack_list(long long b0, long long b1) {
+  return __longlong_as_double((b1 << 19) | (b1 - b0));
+}
+__device__ __forceinline__ long long list_end(double w) { return __double_as_longlong(w) >> 19; }
+__device__ __forceinline__ long long list_size(double w) { return __double_as_longlong(w) & ((1 << 19) - 1); }
+
 __device__ __forceinline__ double s_omega(int kernel, double delta, double L) {
   if (kernel == KER_LINEAR) return delta / L;
   if (kernel == KER_CONST_ONE) return 1.0;
@@ -56,106 +67,157 @@ __device__ __forceinline__ double s_omega(int kernel, double delta, double L) {
   return 0.0;
 }
 
-__device__ __forceinline__ double s_len(const double* p, long long i, long long j, double* d) {
-  d[0] = p[3 * j] - p[3 * i];
-  d[1] = p[3 * j + 1] - p[3 * i + 1];
-  d[2] = p[3 * j + 2] - p[3 * i + 2];
-  return sqrt((d[0] * d[0] + d[1] * d[1]) + d[2] * d[2]);
+// LN lanes share a point. Both phases read a point's bonds with consecutive lanes (the CSR arrays
+// are then read in whole lines) and sum over the lanes in a fixed tree, so results do not depend on
+// the schedule. One thread a point left 958 warps for the chip on a 30,659-point body, each with 122
+// bonds in a row and every load of a bond in a line of its own.
+template <int LN>
+__device__ __forceinline__ double lane_sum(double v) {
+#pragma unroll
+  for (int o = LN / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// the place of a thread: its point, its lane of the point and whether the point exists; lanes of
+// points beyond the last one run along with no bonds
+template <int LN>
+struct Place {
+  long long i, b0, b1;
+  int lane;
+  bool valid;
+  __device__ __forceinline__ Place(const StaticArgs& a) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    i = t / LN;
+    lane = (int)(t % LN);
+    valid = i < a.n;
+    if (!valid) i = 0;
+    b0 = a.off[i];
+    b1 = valid ? a.off[i + 1] : b0;
+  }
+};
+
+__device__ __forceinline__ void s_diff(const double* p, const double (&q)[3], long long j, double (&d)[3]) {
+  d[0] = p[3 * j] - q[0];
+  d[1] = p[3 * j + 1] - q[1];
+  d[2] = p[3 * j + 2] - q[2];
 }
 
 // calc_failure! (ordinary_state_based.jl:107-126), calc_weighted_volume (:176-189),
-// calc_dilatation (:191-204), c1 and c2 (:135-136)
-__global__ void k_static_osb_a(StaticArgs a) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  long long na = 0;
-  double wvol = 0.0;
-  for (long long b = a.off[i]; b < a.off[i + 1]; b++) {
+// calc_dilatation (:191-204), c1 and c2 (:135-136): one pass over the bonds, the dilatation's factor
+// 3 / m taken out of its sum
+template <int LN>
+__global__ void __launch_bounds__(256) k_static_osb_a(StaticArgs a) {
+  const Place<LN> t(a);
+  const long long i = t.i;
+  const double xi[3] = {a.x[3 * i], a.x[3 * i + 1], a.x[3 * i + 2]};
+  const double Xi[3] = {a.X[3 * i], a.X[3 * i + 1], a.X[3 * i + 2]};
+  const double thr = fail_threshold(a.epsc);
+  int na = 0;
+  double m = 0.0, th = 0.0;
+#pragma unroll 2
+  for (long long b = t.b0 + t.lane; b < t.b1; b += LN) {
     const long long j = a.nbr[b];
+    const double L = a.L[b];
+    unsigned act = a.bond_active[b];
     double d[3], D[3];
-    const double l = s_len(a.x, i, j, d);
-    const double eps = (l - a.L[b]) / a.L[b];
-    if (eps > a.epsc && a.fail_permit[b]) a.bond_active[b] = 0;
-    na += a.bond_active[b];
-    s_len(a.X, i, j, D);
-    const double om = a.bond_active[b] ? s_omega(a.kernel, a.delta, a.L[b]) : 0.0;
-    wvol += om * 1.0 * ((D[0] * D[0] + D[1] * D[1]) + D[2] * D[2]) * a.vol[j];
-  }
-  double dil = 0.0, c1 = 0.0, c2 = 0.0;
-  if (wvol != 0.0) {
-    const double c1d = 3.0 / wvol;
-    for (long long b = a.off[i]; b < a.off[i + 1]; b++) {
-      const long long j = a.nbr[b];
-      double d[3];
-      const double l = s_len(a.x, i, j, d);
-      const double om = a.bond_active[b] ? s_omega(a.kernel, a.delta, a.L[b]) : 0.0;
-      dil += om * 1.0 * c1d * a.L[b] * (l - a.L[b]) * a.vol[j];
+    s_diff(a.x, xi, j, d);
+    s_diff(a.X, Xi, j, D);
+    const double l2 = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2];
+    const double e = sqrt_of(l2, rsqrt3(l2)) - L;
+    if (!(L > 0 && e < thr * L) && (sqrt(l2) - L) / L > a.epsc && a.fail_permit[b]) {
+      a.bond_active[b] = 0;
+      act = 0;
     }
-    c1 = 15.0 * a.G / wvol;
-    c2 = dil * (3.0 * a.K / wvol - c1 / 3.0);
+    na += (int)act;
+    const double w = act ? s_omega(a.kernel, a.delta, L) * a.vol[j] : 0.0;
+    m = fma(w, (D[0] * D[0] + D[1] * D[1]) + D[2] * D[2], m);
+    th = fma(w * L, e, th);
   }
-  a.state[i] = make_double4(c1, c2, wvol, dil);
+  m = lane_sum<LN>(m);
+  th = lane_sum<LN>(th);
+#pragma unroll
+  for (int o = LN / 2; o > 0; o >>= 1) na += __shfl_xor_sync(0xffffffffu, na, o);
+  if (!t.valid || t.lane) return;
+  double c1 = 0.0, c2 = 0.0;
+  if (m != 0.0) {
+    c1 = 15.0 * a.G / m;
+    c2 = 3.0 / m * th * (3.0 * a.K / m - c1 / 3.0);
+  }
+  a.state[i] = make_double4(c1, c2, a.vol[i], pack_list(t.b0, t.b1));
   a.n_active[i] = na;
 }
 
-// position of point i in the sorted bond list of point j (the reverse bond j -> i), or -1
-__device__ __forceinline__ long long s_reverse(const StaticArgs& a, long long j, long long i) {
-  long long lo = a.off[j], hi = a.off[j + 1];
+// position of point i in the sorted bond list of point j at [lo, hi) (the reverse bond j -> i), or -1;
+// k: the bond's place in the list of i. In a body whose points lie alike the reverse of a list's k-th
+// bond is the k-th from the end of the other list: that place is tried first.
+__device__ __forceinline__ long long s_reverse(const StaticArgs& a, long long lo, long long hi, long long i,
+                                               long long k) {
+  const long long end = hi, g = hi - 1 - k;
+  if (g >= lo) {
+    const int q = a.nbr[g];
+    if (q == i) return g;
+    if (q < i) lo = g + 1; else hi = g;
+  }
   while (lo < hi) {
     const long long mid = (lo + hi) >> 1;
     if (a.nbr[mid] < i) lo = mid + 1; else hi = mid;
   }
-  return (lo < a.off[j + 1] && a.nbr[lo] == i) ? lo : -1;
+  return (lo < end && a.nbr[lo] == i) ? lo : -1;
 }
 
-// force_density_point! (ordinary_state_based.jl:128-149) gathered in the serial order of the
-// scattered terms: neighbours j < i, the own bonds, neighbours j > i (sorted bond lists). The
-// term of neighbour j is the one its own loop scatters (b_j's bond j -> i: its bond state and
-// its length), so bond states need not be the same in both directions.
-__global__ void k_static_osb_b(StaticArgs a) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
+// force_density_point! (ordinary_state_based.jl:128-149), gathered: a bond's own term and the one
+// that its neighbour's loop scatters into i (of the bond j -> i: its bond state and its length), so
+// bond states need not be the same in both directions.
+template <int LN>
+__global__ void __launch_bounds__(256) k_static_osb_b(StaticArgs a) {
+  const Place<LN> t(a);
+  const long long i = t.i;
   const double4 ci = a.state[i];
-  double bx = 0.0, by = 0.0, bz = 0.0;
-  const long long b0 = a.off[i], b1 = a.off[i + 1];
-  auto nbr_term = [&](long long b) {
+  const double xi[3] = {a.x[3 * i], a.x[3 * i + 1], a.x[3 * i + 2]};
+  const bool own = ci.x != 0.0 || ci.y != 0.0;
+  double f[3] = {0.0, 0.0, 0.0};
+#pragma unroll 2
+  for (long long b = t.b0 + t.lane; b < t.b1; b += LN) {
     const long long j = a.nbr[b];
+    const double L = a.L[b];
     const double4 cj = a.state[j];
-    if (cj.z == 0.0) return;
-    const long long r = s_reverse(a, j, i);
-    if (r < 0) return;  // j has no bond to i: nothing is scattered into i
     double d[3];
-    const double l = s_len(a.x, j, i, d);
-    const double Lr = a.L[r];
-    const double om = a.bond_active[r] ? s_omega(a.kernel, a.delta, Lr) : 0.0;
-    const double s = om * 1.0 * (cj.y * Lr + cj.x * (l - Lr)) / l;
-    bx += -(s * d[0]) * a.vol[j];
-    by += -(s * d[1]) * a.vol[j];
-    bz += -(s * d[2]) * a.vol[j];
-  };
-  long long split = b0;
-  while (split < b1 && a.nbr[split] < i) split++;
-  for (long long b = b0; b < split; b++) nbr_term(b);
-  if (ci.z != 0.0)
-    for (long long b = b0; b < b1; b++) {
-      const long long j = a.nbr[b];
-      double d[3];
-      const double l = s_len(a.x, i, j, d);
-      const double om = a.bond_active[b] ? s_omega(a.kernel, a.delta, a.L[b]) : 0.0;
-      const double s = om * 1.0 * (ci.y * a.L[b] + ci.x * (l - a.L[b])) / l;
-      bx += s * d[0] * a.vol[j];
-      by += s * d[1] * a.vol[j];
-      bz += s * d[2] * a.vol[j];
+    s_diff(a.x, xi, j, d);
+    const double l2 = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2];
+    const double rl = rsqrt3(l2), l = sqrt_of(l2, rl);
+    const double om = s_omega(a.kernel, a.delta, L);
+    double s = (a.bond_active[b] ? om : 0.0) * (ci.y * L + ci.x * (l - L));
+    const long long end = list_end(cj.w), r = s_reverse(a, end - list_size(cj.w), end, i, b - t.b0);
+    if (r >= 0) {  // else j scatters nothing into i
+      const double Lr = a.L[r];
+      const double omr = !a.bond_active[r] ? 0.0 : (Lr == L ? om : s_omega(a.kernel, a.delta, Lr));
+      s += omr * (cj.y * Lr + cj.x * (l - Lr));
     }
-  for (long long b = split; b < b1; b++) nbr_term(b);
-  a.b_int[3 * i] = bx;
-  a.b_int[3 * i + 1] = by;
-  a.b_int[3 * i + 2] = bz;
+    // neither point has bonds left: no force, whatever the bond's length
+    if (!(own || (r >= 0 && (cj.x != 0.0 || cj.y != 0.0)))) continue;
+    s *= rl * cj.z;
+    f[0] = fma(s, d[0], f[0]);
+    f[1] = fma(s, d[1], f[1]);
+    f[2] = fma(s, d[2], f[2]);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++) f[c] = lane_sum<LN>(f[c]);
+  if (!t.valid || t.lane) return;
+  a.b_int[3 * i] = f[0];
+  a.b_int[3 * i + 1] = f[1];
+  a.b_int[3 * i + 2] = f[2];
 }
 
 }  // namespace pd
 
 using namespace pd;
+
+template <int LN>
+static void launch_static(const StaticArgs& a, cudaStream_t s) {
+  const int blocks = (int)((a.n * LN + 255) / 256);
+  k_static_osb_a<LN><<<blocks, 256, 0, s>>>(a);
+  k_static_osb_b<LN><<<blocks, 256, 0, s>>>(a);
+}
 
 static thread_local std::string g_static_err;
 
@@ -269,9 +331,12 @@ extern "C" pd_status pd_osb_force_static(int64_t n, const double* ref_position, 
   a.n_active = reinterpret_cast<long long*>(n_active);
   a.state = (double4*)state;
   cudaStream_t s = (cudaStream_t)stream;
-  const int blocks = (int)((n + 127) / 128);
-  k_static_osb_a<<<blocks, 128, 0, s>>>(a);
-  k_static_osb_b<<<blocks, 128, 0, s>>>(a);
+  // Small bodies want a point's bonds spread over many lanes, large ones few idle lanes and short sums
+  // over lanes. us a call with 32 / 16 / 8 lanes: 1,380 points 42 / 50 / 70, 4,095 44 / 54 / 76, 9,768
+  // 76 / 75 / 84, 30,659 168 / 150 / 158, 47,196 294 / 243 / 233, 147,420 1000 / 815 / 730
+  if (n <= (1 << 13)) launch_static<32>(a, s);
+  else if (n <= 5 * (1 << 13)) launch_static<16>(a, s);
+  else launch_static<8>(a, s);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     g_static_err = std::string("kernel launch: ") + cudaGetErrorString(e);
