@@ -22,6 +22,7 @@
 //                  as an FP32 bond sweep (one gather of v per bond);
 //   learned        B_i = P_i (I + D_i) with per-point corrections D from the message-passing
 //                  network, used alone or in the polynomial.
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstring>
@@ -47,7 +48,8 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// part[q * gridDim.x + block] = sum over the block's rows of V_q[r] w[r], q < k
+// part[q * gridDim.x + block] = sum over the block's rows of V_q[r] w[r], for the four vectors q of
+// blockIdx.y
 __global__ void __launch_bounds__(NK_TPB) k_mdot(const double* __restrict__ V, int k, long long ld,
                                                  const double* __restrict__ w, long long n,
                                                  double* __restrict__ part) {
@@ -55,27 +57,24 @@ __global__ void __launch_bounds__(NK_TPB) k_mdot(const double* __restrict__ V, i
   const long long chunk = ((n + gridDim.x - 1) / gridDim.x + 31) / 32 * 32;
   const long long r0 = (long long)blockIdx.x * chunk;
   const long long r1 = r0 + chunk < n ? r0 + chunk : n;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int q0 = 0; q0 < k; q0 += 4) {
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (long long r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-      const double wr = w[r];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q0 = 4 * blockIdx.y;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  for (long long r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
+    const double wr = w[r];
 #pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (q0 + u < k) acc[u] += V[(long long)(q0 + u) * ld + r] * wr;
-    }
+    for (int u = 0; u < 4; u++)
+      if (q0 + u < k) acc[u] += V[(long long)(q0 + u) * ld + r] * wr;
+  }
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const double s = warp_sum(acc[u]);
-      if (lane == 0) red[warp][u] = s;
-    }
-    __syncthreads();
-    if (threadIdx.x < 4 && q0 + (int)threadIdx.x < k) {
-      double s = 0.0;
-      for (int wp = 0; wp < NK_TPB / 32; wp++) s += red[wp][threadIdx.x];
-      part[(long long)(q0 + threadIdx.x) * gridDim.x + blockIdx.x] = s;
-    }
-    __syncthreads();
+  for (int u = 0; u < 4; u++) {
+    const double s = warp_sum(acc[u]);
+    if (lane == 0) red[warp][u] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < 4 && q0 + (int)threadIdx.x < k) {
+    double s = 0.0;
+    for (int wp = 0; wp < NK_TPB / 32; wp++) s += red[wp][threadIdx.x];
+    part[(long long)(q0 + threadIdx.x) * gridDim.x + blockIdx.x] = s;
   }
 }
 
@@ -99,6 +98,7 @@ __global__ void __launch_bounds__(NK_TPB) k_mupd(double* __restrict__ w, const d
   for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n;
        r += (long long)gridDim.x * blockDim.x) {
     double acc = 0.0;
+#pragma unroll 8
     for (int q = 0; q < k; q++) acc += cs[q] * V[(long long)q * ld + r];
     w[r] = w[r] + sgn * acc;
   }
@@ -240,26 +240,49 @@ __device__ __forceinline__ double bb_c(const DevBody& d, const DevParam& Pi, int
 // P_i = J_ii^-1 with J_ii = -V_i sum_j V_j c [(1/L - 1/l) I + d d^T / l^3] over the active
 // bonds (the derivative of the bond force of bond_based.jl:146-180 with respect to u_i);
 // rows and columns of constrained dofs are the identity.
-__global__ void k_bj_blocks(DevBody d, const unsigned char* __restrict__ cmask, float* __restrict__ P) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= d.n) return;
-  const int cnt = (int)(d.off[i + 1] - d.off[i]);
+// A block takes 32 points, eight threads a point: thread p of a point takes its bonds p, p + 8 and so
+// on, and the eight sums of the six entries are added in their order (one thread a point walked 122 bonds: 176 us
+// on a 7,200-point beam).
+__global__ void __launch_bounds__(256) k_bj_blocks(DevBody d, const unsigned char* __restrict__ cmask,
+                                                   float* __restrict__ P) {
+  if (d.n == 0) return;
+  __shared__ double sh[8][6][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long q = (long long)blockIdx.x * 32 + lane;
+  const bool valid = q < d.n;
+  const long long i = valid ? point_at(d, q) : 0;
+  const int cnt = valid ? (int)(d.off[i + 1] - d.off[i]) : 0;
   const double4 xi = d.cur[i];
   const DevParam& Pi = d.params[d.meta[i] & META_PID_MASK];
-  double J[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int k = 0; k < cnt; k++) {
+  double S[6] = {0, 0, 0, 0, 0, 0};  // xx, yy, zz, xy, xz, yz
+  for (int k = w; k < cnt; k += 8) {
     const long long b = bond_slot(d, i, k);
     if (!bond_bit(d.bits, b)) continue;
     const int j = d.nbr[b];
     const double L = fabs(d.len64[b]);
     const double4 xj = d.cur[j];
-    const double dv[3] = {xj.x - xi.x, xj.y - xi.y, xj.z - xi.z};
-    const double l = sqrt((dv[0] * dv[0] + dv[1] * dv[1]) + dv[2] * dv[2]);
+    const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
+    const double l = sqrt((dx * dx + dy * dy) + dz * dz);
     const double s = bb_c(d, Pi, j) * xj.w * xi.w;
     const double a = s * (1.0 / L - 1.0 / l), g = s / (l * l * l);
-    for (int c = 0; c < 3; c++)
-      for (int r = 0; r < 3; r++) J[r + 3 * c] -= (r == c ? a : 0.0) + g * dv[r] * dv[c];
+    S[0] -= a + g * dx * dx;
+    S[1] -= a + g * dy * dy;
+    S[2] -= a + g * dz * dz;
+    S[3] -= g * dx * dy;
+    S[4] -= g * dx * dz;
+    S[5] -= g * dy * dz;
   }
+#pragma unroll
+  for (int c = 0; c < 6; c++) sh[w][c][lane] = S[c];
+  __syncthreads();
+  if (w != 0 || !valid) return;
+#pragma unroll
+  for (int c = 0; c < 6; c++) {
+    S[c] = sh[0][c][lane];
+#pragma unroll
+    for (int p = 1; p < 8; p++) S[c] += sh[p][c][lane];
+  }
+  double J[9] = {S[0], S[3], S[4], S[3], S[1], S[5], S[4], S[5], S[2]};
   for (int a = 0; a < 3; a++) {
     if (!cmask[3 * i + a]) continue;
     for (int b = 0; b < 3; b++) J[a + 3 * b] = J[b + 3 * a] = (a == b) ? 1.0 : 0.0;
@@ -324,48 +347,71 @@ __global__ void k_pack4(float4* __restrict__ kx, const double* __restrict__ v, l
 // stiffness K0 of the reference configuration, in FP32 from FP32 copies of the reference
 // positions (xi = X_j - X_i, L = |xi|: the bond arrays are read for the neighbour and the
 // bond bit only, one 32-byte gather per bond); constrained rows 0
-template <int G>
+// W warps share a slice: warp p takes the rows 4 p .. 4 p + 3, 4 p + 4 W .. and so on, and the
+// warps' sums are added in their order. One warp a slice walked 122 rows of dependent loads, whatever
+// the size of the body: 62 us a product on a 7,200-point beam, 13 so.
+template <int G, int W>
 __global__ void __launch_bounds__(256) k_k0(DevBody d, const float4* __restrict__ kx,
                                             const unsigned char* __restrict__ cmask,
                                             double* __restrict__ out) {
-  PD_SLICE_LOOP(G) {
-    PD_SLICE_SETUP
-    float ax = 0.f, ay = 0.f, az = 0.f;
-    const float4 Xi = valid ? kx[2 * i] : make_float4(0, 0, 0, 0);
-    const float4 vi = valid ? kx[2 * i + 1] : make_float4(0, 0, 0, 0);
-    const DevParam& Pi = d.params[valid ? (d.meta[i] & META_PID_MASK) : 0];
-    const float ci = (float)Pi.bc;
-    const int self = valid ? (int)i : 0;
-    // two rows per iteration: two independent neighbour gathers in flight per lane
-    for (int r = 0; r < rows; r += 2) {
-      const int k0 = r * G + gl, k1 = k0 + G;
-      const long long b0 = sbase + (long long)r * 32 + lane, b1 = b0 + 32;
-      const bool a0 = k0 < cnt && bond_bit(d.bits, b0);
-      const bool a1 = r + 1 < rows && k1 < cnt && bond_bit(d.bits, b1);
-      const int j0 = a0 ? __ldg(d.nbr + b0) : self;
-      const int j1 = a1 ? __ldg(d.nbr + b1) : self;
-      const float4 X0 = __ldg(kx + 2 * j0), v0 = __ldg(kx + 2 * j0 + 1);
-      const float4 X1 = __ldg(kx + 2 * j1), v1 = __ldg(kx + 2 * j1 + 1);
+  constexpr int P = 32 / G;
+  __shared__ float sh[8][3][32];
+  const int wb = threadIdx.x >> 5, w = wb % W, lane = threadIdx.x & 31, gl = lane % G;
+  const long long s = (long long)blockIdx.x * (8 / W) + wb / W;
+  const bool live = s < d.nslices;
+  const long long place = s * P + lane / G;
+  const bool valid = live && place < d.n;
+  const long long i = valid ? point_at(d, place) : 0;
+  const long long sbase = live ? d.soff[s] : 0;
+  const int rows = live ? (int)((d.soff[s + 1] - sbase) >> 5) : 0;
+  const int cnt = valid ? (int)(d.off[i + 1] - d.off[i]) : 0;
+  const float4 Xi = kx[2 * i], vi = kx[2 * i + 1];
+  const DevParam& Pi = d.params[d.meta[i] & META_PID_MASK];
+  const float ci = (float)Pi.bc;
+  float f[3] = {0.f, 0.f, 0.f};
+  for (int r0 = 4 * w; r0 < rows; r0 += 4 * W) {
+    int j[4];
+    float4 X[4], v[4];
 #pragma unroll
-      for (int u = 0; u < 2; u++) {
-        const bool a = u ? a1 : a0;
-        if (!a) continue;
-        const float4 Xj = u ? X1 : X0, vj = u ? v1 : v0;
-        const float ex = Xj.x - Xi.x, ey = Xj.y - Xi.y, ez = Xj.z - Xi.z;
-        const float L2 = (ex * ex + ey * ey) + ez * ez;
-        const float c = d.multi ? (float)bb_c(d, Pi, u ? j1 : j0) : ci;
-        const float kk = c * Xj.w / (L2 * sqrtf(L2));
-        const float pr = kk * (ex * (vj.x - vi.x) + ey * (vj.y - vi.y) + ez * (vj.z - vi.z));
-        ax += pr * ex; ay += pr * ey; az += pr * ez;
-      }
+    for (int u = 0; u < 4; u++) {
+      const int r = r0 + u;
+      const long long b = sbase + (long long)r * 32 + lane;
+      j[u] = r < rows && r * G + gl < cnt && bond_bit(d.bits, b) ? __ldg(d.nbr + b) : -1;
     }
-    if (G > 1) { ax = group_sum<G>(ax); ay = group_sum<G>(ay); az = group_sum<G>(az); }
-    if (valid && gl == 0) {
-      const double V = Xi.w;
-      out[3 * i] = cmask[3 * i] ? 0.0 : (double)ax * V;
-      out[3 * i + 1] = cmask[3 * i + 1] ? 0.0 : (double)ay * V;
-      out[3 * i + 2] = cmask[3 * i + 2] ? 0.0 : (double)az * V;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const long long q = 2 * (j[u] < 0 ? i : (long long)j[u]);
+      X[u] = __ldg(kx + q);
+      v[u] = __ldg(kx + q + 1);
     }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      if (j[u] < 0) continue;
+      const float ex = X[u].x - Xi.x, ey = X[u].y - Xi.y, ez = X[u].z - Xi.z;
+      const float L2 = (ex * ex + ey * ey) + ez * ez;
+      const float c = d.multi ? (float)bb_c(d, Pi, j[u]) : ci;
+      const float kk = c * X[u].w / (L2 * sqrtf(L2));
+      const float pr = kk * (ex * (v[u].x - vi.x) + ey * (v[u].y - vi.y) + ez * (v[u].z - vi.z));
+      f[0] += pr * ex;
+      f[1] += pr * ey;
+      f[2] += pr * ez;
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++) f[c] = G > 1 ? group_sum<G>(f[c]) : f[c];
+  if constexpr (W > 1) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) sh[wb][c][lane] = f[c];
+    __syncthreads();
+    if (w < 3 && valid && gl == 0) {
+      float a = 0.f;
+#pragma unroll
+      for (int q = 0; q < W; q++) a += sh[wb - w + q][w][lane];
+      out[3 * i + w] = cmask[3 * i + w] ? 0.0 : (double)a * Xi.w;
+    }
+  } else if (valid && gl == 0) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) out[3 * i + c] = cmask[3 * i + c] ? 0.0 : (double)f[c] * Xi.w;
   }
 }
 
@@ -438,8 +484,11 @@ static pd_status nk_zbasis(pd_handle* h) {
 // out[0..k) = V_q . w (V_q = V + q ld)
 static void nk_dots(pd_handle* h, const double* V, int k, const double* w, double* out) {
   NKState* S = h->nk;
-  k_mdot<<<NK_NB, NK_TPB, 0, h->stream>>>(V, k, S->ld, w, S->ndof, S->part);
-  k_reduce<<<(k + 7) / 8, 256, 0, h->stream>>>(S->part, k, NK_NB, out);
+  // a row a thread until there are NK_NB blocks: with 592 blocks of 32 rows on the 17,820-row beam the
+  // second kernel read eight times the partial sums it does now
+  const int nb = (int)std::min<long long>(std::max<long long>((S->ndof + NK_TPB - 1) / NK_TPB, 1), NK_NB);
+  k_mdot<<<dim3(nb, (k + 3) / 4), NK_TPB, 0, h->stream>>>(V, k, S->ld, w, S->ndof, S->part);
+  k_reduce<<<(k + 7) / 8, 256, 0, h->stream>>>(S->part, k, nb, out);
   h->launches += 2;
 }
 
@@ -479,21 +528,23 @@ static void nk_matvec(pd_handle* h, const pd_nk_params& p, const double* v, doub
   if (st) st->matvecs++;
 }
 
+#define PD_K0_CASE(G, W) \
+  case G: k_k0<G, W><<<(unsigned)((h->d.nslices * W + 7) / 8), 256, 0, h->stream>>>( \
+      h->d, S->kx, S->cmask, out); break;
+#define PD_DISPATCH_K0(W) \
+  switch (h->d.lg) { \
+    PD_K0_CASE(1, W) PD_K0_CASE(2, W) PD_K0_CASE(4, W) PD_K0_CASE(8, W) PD_K0_CASE(16, W) \
+    PD_K0_CASE(32, W) \
+  }
 static void nk_k0(pd_handle* h, const double* v, double* out) {
   NKState* S = h->nk;
+  if (h->n == 0) return;
   k_pack4<<<nk_grid(h->n, 256), 256, 0, h->stream>>>(S->kx, v, h->n);
-  long long blocks = (h->d.nslices + 7) / 8;
-  if (blocks < 1) blocks = 1;
-  if (PD_GRID_BLOCKS_PER_SM > 0 && blocks > 148LL * PD_GRID_BLOCKS_PER_SM)
-    blocks = 148LL * PD_GRID_BLOCKS_PER_SM;
-  const int grid = (int)blocks;
-  switch (h->d.lg) {
-    case 1: k_k0<1><<<grid, 256, 0, h->stream>>>(h->d, S->kx, S->cmask, out); break;
-    case 2: k_k0<2><<<grid, 256, 0, h->stream>>>(h->d, S->kx, S->cmask, out); break;
-    case 4: k_k0<4><<<grid, 256, 0, h->stream>>>(h->d, S->kx, S->cmask, out); break;
-    case 8: k_k0<8><<<grid, 256, 0, h->stream>>>(h->d, S->kx, S->cmask, out); break;
-    case 16: k_k0<16><<<grid, 256, 0, h->stream>>>(h->d, S->kx, S->cmask, out); break;
-    default: k_k0<32><<<grid, 256, 0, h->stream>>>(h->d, S->kx, S->cmask, out); break;
+  // eight warps a slice until the slices fill the chip by themselves (24 warps per SM)
+  if (h->d.nslices <= 148LL * 24) {
+    PD_DISPATCH_K0(8);
+  } else {
+    PD_DISPATCH_K0(1);
   }
   h->launches += 2;
 }
@@ -513,7 +564,7 @@ static pd_status nk_prepare_pc(pd_handle* h, int pc) {
   NKState* S = h->nk;
   PD_TRY(nk_check_pc(h, pc));
   if (pc == PD_PC_NONE) return PD_OK;
-  k_bj_blocks<<<nk_grid(h->n, 128), 128, 0, h->stream>>>(h->d, S->cmask, S->P);
+  k_bj_blocks<<<(int)std::max<long long>((h->n + 31) / 32, 1), 256, 0, h->stream>>>(h->d, S->cmask, S->P);
   h->launches++;
   return PD_OK;
 }
@@ -848,7 +899,7 @@ void nk_dots_dev(pd_handle* h, const double* V, int k, const double* w, double* 
 }
 void nk_apply_k0(pd_handle* h, const double* v, double* out) { nk_k0(h, v, out); }
 void nk_compute_blocks(pd_handle* h) {
-  k_bj_blocks<<<nk_grid(h->n, 128), 128, 0, h->stream>>>(h->d, h->nk->cmask, h->nk->P);
+  k_bj_blocks<<<(int)std::max<long long>((h->n + 31) / 32, 1), 256, 0, h->stream>>>(h->d, h->nk->cmask, h->nk->P);
   h->launches++;
 }
 void nk_apply_blocks(pd_handle* h, const float* D, const double* v, double a, const double* s,
