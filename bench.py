@@ -56,10 +56,17 @@ DR_STRAIN = 5e-5
 # v_half_old read, v_half, v, v_half_old, b_int_old written)
 # (FP64: 128 + 176 B; FP32: b_int is 12 B, 116 + 164 B)
 B_DR_POINT = {"fp64": 304.0, "fp32": 280.0}
-# algorithmic bytes (FP32-compensated form): per directed bond nbr 4 + xi 12 + L 4 + 1/8 bit;
-# per point 140 (u, v FP64 read+write, own u, b_ext/BC, parameter id, damage) + 8 for OSB
+# algorithmic bytes (FP32-compensated form): per directed bond the neighbour's place in its tile 2 +
+# class of its reference vector 1 + 1/8 bit (FP64 BB and OSB: place 2 + length 8 + 1/8 bit; FP64 CMat
+# nbr 4 + gathered X 24 + length 8 + 1/8 bit; energy correction, which runs without tiles: nbr 4 + xi
+# 12 + L 4 + factor 4 (FP64: 8) + 1/8 bit); per point 140 (u, v FP64 read+write, own u, b_ext/BC, parameter id, damage) + 8 for OSB
 # (m, theta) + 72 for CMat (F, P K^-1) + 24 with ZEMWan (the symmetric stiffness C : K^-1)
-B_BOND = {"fp32": 20.125, "fp64": 36.125}
+def bond_bytes(prec, mat, energy=False):
+    if energy:
+        return {"fp32": 24.125, "fp64": 44.125}[prec]
+    return 3.125 if prec == "fp32" else 36.125 if mat.startswith("C") else 10.125
+
+
 B_POINT = {"fp32": 140.0, "fp64": 184.0}
 B_POINT_EXTRA = {"BB": 0.0, "OSB": 8.0, "C": 72.0, "CW": 96.0}
 # steps of the legs beside the timed run (per-kernel events, end to end): at most this many
@@ -646,7 +653,7 @@ def run_dr(args, rank, world, local, dist):
     # roofline: the force kernels of a step (OSB: phases A and B each stream every bond once)
     n_phase = 1 if mat == "BB" else 2
     pt = {"fp32": 64 + 8 + 16 + 4 + 4, "fp64": 128 + 8 + 32 + 4 + 4}[prec]
-    force_bytes = n_phase * (n_bonds * B_BOND[prec] + n_pts * pt)
+    force_bytes = n_phase * (n_bonds * bond_bytes(prec, mat) + n_pts * pt)
     peak, peak_kind = load_peaks()
     force_ms = ms_force / args.steps
     achieved = force_bytes / (force_ms / 1e3) / 1e9
@@ -749,7 +756,7 @@ def run_halo(args, rank, world, local, dist):
     prec = args.precision
     dom = "force_b" if "force_b" in ms else "force_a"
     pt_bytes = {"fp32": 32 + 8 + 16 + 12 + 4, "fp64": 64 + 8 + 32 + 24 + 4}[prec]
-    alg = all_bonds * B_BOND[prec] + rows * pt_bytes
+    alg = all_bonds * bond_bytes(prec, mat) + rows * pt_bytes
     dom_ms = ms[dom] / args.steps
     peak, peak_kind = load_peaks()
     achieved = alg / (dom_ms / 1e3) / 1e9
@@ -1167,13 +1174,13 @@ def main():
     per_kernel = {"phase_a": ms_a / n_launch, "phase_b": ms_b / n_launch}
     dom = max(per_kernel, key=per_kernel.get) if mat != "BB" else "phase_a"
     dom_ms = per_kernel[dom]
-    # bytes a launch of one force phase must move: every bond once (nbr, geometry, state bit)
+    # bytes a launch of one force phase must move: every bond's stream once
     # and its per-point reads / writes
     if prec == "fp32":
         pt_bytes = {"phase_a": 32 + 8 + 16 + 4 + 4, "phase_b": 32 + 8 + 16 + 12 + 4}[dom]
     else:
         pt_bytes = {"phase_a": 64 + 8 + 32 + 4 + 4, "phase_b": 64 + 8 + 32 + 24 + 4}[dom]
-    b_bond = B_BOND[prec] + (({"fp32": 4.0, "fp64": 8.0}[prec]) if args.correction == "energy" else 0.0)
+    b_bond = bond_bytes(prec, mat, args.correction == "energy")
     alg_bytes = n_bonds * b_bond + n_pts * pt_bytes
     achieved = alg_bytes / (dom_ms / 1e3) / 1e9
     # DRAM traffic per launch from the committed ncu capture, scaled by the bond count
@@ -1253,14 +1260,17 @@ def main():
                        "mapping": dict(zip(("group", "block", "pipe"), dev_mapping)),
                        "symmetric_pairs": bool(sym), "graph_steps": gsteps,
                        "l2": ("inputs larger than L2 (bond arrays of "
-                              f"{n_bonds * B_BOND[prec] / 1e9:.1f} GB)" if n_bonds * B_BOND[prec] > 126e6
+                              f"{n_bonds * b_bond / 1e9:.1f} GB)" if n_bonds * b_bond > 126e6
                               else "inputs smaller than L2: the plate job as stated (L2 not flushed)"),
                        "parallelism": f"replicas x{world}"},
-            "roofline": {"bound": "hbm", "kernel": f"{mat.lower()} force {dom}",
+            # on tiles issue slots and shared memory bound the force kernels; the bytes are those of
+            # the stream that they read
+            "roofline": {"bound": "hbm" if args.correction == "energy" else "issue",
+                         "kernel": f"{mat.lower()} force {dom}",
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
                          "traffic_source": "profiles/traffic.json (ncu DRAM counters of both "
-                                           "phases captured on the 8M-point block, per bond)",
+                                           "phases captured on the 1M-point block, per bond)",
                          "alg_bytes_per_launch": alg_bytes, "ms_per_launch": dom_ms},
             "roofline_step": {"achieved": step_achieved, "peak": peak, "frac": step_achieved / peak,
                               "alg_bytes_per_step": step_bytes,
