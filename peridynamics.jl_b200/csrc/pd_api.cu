@@ -284,10 +284,10 @@ static pd_status finish_create(pd_handle* h, int* dnbr_csr, const double* dL, co
       if (h->zem == PD_ZEM_WAN) {
         PD_TRY(dalloc(h, &h->d.C164, 9 * n));
         PD_CUDA(cudaMemsetAsync(h->d.C164, 0, sizeof(double) * 9 * n, h->stream));
-      } else {
-        PD_TRY(dalloc(h, &h->d.cst64, 5 * n));
-        PD_CUDA(cudaMemsetAsync(h->d.cst64, 0, sizeof(double2) * 5 * n, h->stream));
       }
+      const long long planes = h->zem == PD_ZEM_WAN ? 8 : 5;
+      PD_TRY(dalloc(h, &h->d.cst64, planes * n));
+      PD_CUDA(cudaMemsetAsync(h->d.cst64, 0, sizeof(double2) * planes * n, h->stream));
     } else {
       PD_TRY(dalloc(h, &h->d.H32, 9 * n));
       PD_TRY(dalloc(h, &h->d.cst32, 3 * n));

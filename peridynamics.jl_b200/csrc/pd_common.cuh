@@ -121,7 +121,7 @@ struct DevBody {
   float4* ulo;       // FP32 path: {(float)(u - hi), 0}
   double* F64;       // CMat FP64: deformation gradient F (9 per point, column-major)
   double* PK64;      // CMat FP64: P K^-1 (9 per point)
-  double2* cst64;    // CMat FP64, ZEMSilling: phase-B state in five planes of n (pd_math64.cuh)
+  double2* cst64;    // CMat FP64: phase-B state in planes of n (pd_math64.cuh)
   float* H32;        // CMat FP32: displacement gradient H = F - I (9 per point)
   float4* cst32;     // CMat FP32: 3 float4 per point {A (9), beta~, 0, 0}
   // CMat with ZEMWan: the stabilising stiffness C : K^-1 of every point (FP64: 9 per point,

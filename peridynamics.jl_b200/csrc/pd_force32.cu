@@ -17,6 +17,10 @@
 // cancel) and a horizon-scaled shape tensor K' = K / delta^5 (the unscaled det K underflows
 // FP32 for millimetre lattices). The stress formulas are the reference's, rewritten in
 // terms of E = (H + H^T + H^T H) / 2 without cancelling subtractions.
+//
+// Bodies with tiles (one lane per point, bond-stream variants 0, 4 and 5) run pd_tile32.cu; the kernels
+// here serve the other lane groups, ZEMWan's phase B, directed bond states, several parameter sets in
+// phase B and EnergySurfaceCorrection.
 #include "pd_bond32.cuh"
 #include "pd_common.cuh"
 #include "pd_launch.h"

@@ -489,21 +489,24 @@ __global__ void __launch_bounds__(256, MB_CA) k_c_a64f(DevBody d, int kstep) {
 }
 
 // -------------------------------------------------------------------------------------------
-// CMat phase B (correspondence.jl:226-251) for ZEMSilling, symmetric bond states and one
-// parameter set: b_i = sum_j omega V_j ((A_i + A_j) xi + (beta_i + beta_j) du). A killed point
-// holds A = 0 and beta = 0.
+// CMat phase B (correspondence.jl:226-251) for symmetric bond states and one parameter set: b_i =
+// sum_j omega V_j ((A_i + A_j) xi + (S_i + S_j) du), S = beta I for ZEMSilling. A killed point holds
+// A = 0 and S = 0. ZEMWan's 15 values a point take 128 bytes of gathers a bond beside the 64 of the
+// positions (one block an SM, no spills): 73,062 points 588 -> 289 us a step against the kernel that reads
+// F, P K^-1 and C1 of both points, 2,233 points 294 -> 46.
 // -------------------------------------------------------------------------------------------
-template <int G, int W, bool LIN>
-__global__ void __launch_bounds__(256, MB_CB) k_c_b64f(DevBody d, int kstep) {
+template <int G, int W, bool LIN, bool WAN>
+__global__ void __launch_bounds__(256, WAN ? 1 : MB_CB) k_c_b64f(DevBody d, int kstep) {
   if (stopped<W>(d)) return;
   constexpr int RU = RU_CB;
   const Place<G, W> p(d, false);
   const double4 xi = ld4_64(d.cur + p.self), Xi = ld4_64(d.X0 + p.self);
   const double delta = d.params[p.valid ? d.meta[p.self] & META_PID_MASK : 0].delta, rdelta = 1.0 / delta;
   const long long n = d.n;
-  double2 Ai[5];
+  constexpr int NP = WAN ? 8 : 5;
+  double2 Ai[NP];
 #pragma unroll
-  for (int k = 0; k < 5; k++) Ai[k] = d.cst64[k * n + p.self];
+  for (int k = 0; k < NP; k++) Ai[k] = d.cst64[k * n + p.self];
   Totals<W, 3, false> T(p.part, p.lane);
   Rows<G, RU, false, false> nx;
   if (p.part * SEG < p.rows) nx.load(p, p.part * SEG);
@@ -518,19 +521,32 @@ __global__ void __launch_bounds__(256, MB_CB) k_c_b64f(DevBody d, int kstep) {
         const bool a = (c.w[u] >> p.lane) & 1u;
         const int j = a ? c.j[u] : p.self;
         const double4 x = ld_point(d.cur + j), X = ld_point(d.X0 + j);
-        double2 Aj[5];
+        double2 Aj[NP];
 #pragma unroll
-        for (int k = 0; k < 5; k++) Aj[k] = __ldg(d.cst64 + k * n + j);
+        for (int k = 0; k < NP; k++) Aj[k] = __ldg(d.cst64 + k * n + j);
         if (u == 0 && nr < p.rows) nx.load(p, nr);
         const double L = fabs(c.L[u]);
         const double DX = X.x - Xi.x, DY = X.y - Xi.y, DZ = X.z - Xi.z;
-        const double b = Ai[4].y + Aj[4].y;
         const double ux = (x.x - xi.x) - DX, uy = (x.y - xi.y) - DY, uz = (x.z - xi.z) - DZ;
         const double om = LIN ? delta * rcp3(L) : omega64(d.kernel, delta, rdelta, L);
         const double f = a ? om * x.w : 0.0;
-        const double t0 = fma(Ai[0].x + Aj[0].x, DX, fma(Ai[1].y + Aj[1].y, DY, fma(Ai[3].x + Aj[3].x, DZ, b * ux)));
-        const double t1 = fma(Ai[0].y + Aj[0].y, DX, fma(Ai[2].x + Aj[2].x, DY, fma(Ai[3].y + Aj[3].y, DZ, b * uy)));
-        const double t2 = fma(Ai[1].x + Aj[1].x, DX, fma(Ai[2].y + Aj[2].y, DY, fma(Ai[4].x + Aj[4].x, DZ, b * uz)));
+        // S du
+        double s0, s1, s2;
+        if constexpr (WAN) {
+          const double xx = Ai[4].y + Aj[4].y, yy = Ai[5].x + Aj[5].x, zz = Ai[5].y + Aj[5].y;
+          const double xy = Ai[6].x + Aj[6].x, xz = Ai[6].y + Aj[6].y, yz = Ai[7].x + Aj[7].x;
+          s0 = fma(xx, ux, fma(xy, uy, xz * uz));
+          s1 = fma(xy, ux, fma(yy, uy, yz * uz));
+          s2 = fma(xz, ux, fma(yz, uy, zz * uz));
+        } else {
+          const double b = Ai[4].y + Aj[4].y;
+          s0 = b * ux;
+          s1 = b * uy;
+          s2 = b * uz;
+        }
+        const double t0 = fma(Ai[0].x + Aj[0].x, DX, fma(Ai[1].y + Aj[1].y, DY, fma(Ai[3].x + Aj[3].x, DZ, s0)));
+        const double t1 = fma(Ai[0].y + Aj[0].y, DX, fma(Ai[2].x + Aj[2].x, DY, fma(Ai[3].y + Aj[3].y, DZ, s1)));
+        const double t2 = fma(Ai[1].x + Aj[1].x, DX, fma(Ai[2].y + Aj[2].y, DY, fma(Ai[4].x + Aj[4].x, DZ, s2)));
         seg[0] = fma(f, t0, seg[0]);
         seg[1] = fma(f, t1, seg[1]);
         seg[2] = fma(f, t2, seg[2]);
@@ -555,7 +571,8 @@ __global__ void k_c_state_rows(DevBody d, const int* rows, long long n) {
   const long long i = rows[r];
   if (i < 0 || i >= d.n) return;
   const unsigned meta = d.meta[i];
-  c_state64(d, i, meta & META_KILLED, d.params[meta & META_PID_MASK].beta, d.F64 + 9 * i, d.PK64 + 9 * i);
+  c_state64(d, i, meta & META_KILLED, d.params[meta & META_PID_MASK].beta, d.F64 + 9 * i, d.PK64 + 9 * i,
+            d.C164 ? d.C164 + 9 * i : nullptr);
 }
 
 void launch_c_state_rows(const DevBody& d, const int* rows, long long n, cudaStream_t s) {
@@ -613,7 +630,7 @@ static Shape shape_for(const DevBody& d, const LaunchCfg& c, int W) {
 // phase B (every BB evaluation and phase A run here)
 bool fast64_supported(const DevBody& d) {
   if (!d.sym || d.multi) return false;  // reverse bonds, bond-averaged parameters
-  return d.material == MAT_OSB || d.zem != ZEM_WAN;
+  return true;
 }
 
 template <bool ESC>
@@ -631,7 +648,8 @@ static void launch_osb64f(const DevBody& d, const Shape& q, int W, int kstep, in
 template <bool LIN>
 static void launch_c64f(const DevBody& d, const Shape& q, int W, int kstep, int phase, cudaStream_t s) {
   if (phase == 1) { PD_DISPATCH_GW(d, W, (k_c_a64f<GG, WW, LIN><<<q.grid, q.block, 0, s>>>(d, kstep))) }
-  else { PD_DISPATCH_GW(d, W, (k_c_b64f<GG, WW, LIN><<<q.grid, q.block, 0, s>>>(d, kstep))) }
+  else if (d.zem == ZEM_WAN) { PD_DISPATCH_GW(d, W, (k_c_b64f<GG, WW, LIN, true><<<q.grid, q.block, 0, s>>>(d, kstep))) }
+  else { PD_DISPATCH_GW(d, W, (k_c_b64f<GG, WW, LIN, false><<<q.grid, q.block, 0, s>>>(d, kstep))) }
 }
 
 void launch_force64_fast(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s) {

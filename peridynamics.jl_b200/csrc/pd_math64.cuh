@@ -117,12 +117,31 @@ static __device__ void pk1_64(int cmodel, const DevParam& p, const double* F, do
   matmul3(F, S, P);
 }
 
-// The phase-B state of a point for the kernels off the serial order: A = P K^-1 - beta (F - I)
-// and beta in five planes {A0 A1}, {A2 A3}, {A4 A5}, {A6 A7}, {A8 beta} (column-major A); zero for
-// a killed point.
+// The phase-B state of a point for the kernels off the serial order: A = P K^-1 - S (F - I) and the
+// stabilising stiffness S, in planes of n; zero for a killed point. ZEMSilling, S = beta I: five planes
+// {A0 A1}, {A2 A3}, {A4 A5}, {A6 A7}, {A8 beta} (column-major A). ZEMWan, S = C1 = C : K^-1 (symmetric):
+// {A8 Sxx}, {Syy Szz}, {Sxy Sxz}, {Syz 0} follow the first four.
 __device__ __forceinline__ void c_state64(const DevBody& d, long long i, bool killed, double beta,
-                                          const double* F, const double* PK) {
-  if (d.cst64 == nullptr) return;
+                                          const double* F, const double* PK, const double* C1) {
+  if (d.zem == ZEM_WAN) {
+    double A[16];
+    for (int c = 0; c < 3; c++)
+      for (int r = 0; r < 3; r++) {
+        double s = 0.0;
+        for (int k = 0; k < 3; k++) s += C1[r + 3 * k] * (k == c ? F[k + 3 * c] - 1.0 : F[k + 3 * c]);
+        A[r + 3 * c] = PK[r + 3 * c] - s;
+      }
+    A[9] = C1[0];
+    A[10] = C1[4];
+    A[11] = C1[8];
+    A[12] = 0.5 * (C1[1] + C1[3]);
+    A[13] = 0.5 * (C1[2] + C1[6]);
+    A[14] = 0.5 * (C1[5] + C1[7]);
+    A[15] = 0.0;
+    for (int k = 0; k < 8; k++)
+      d.cst64[k * d.n + i] = killed ? make_double2(0.0, 0.0) : make_double2(A[2 * k], A[2 * k + 1]);
+    return;
+  }
   double A[10];
   for (int q = 0; q < 9; q++)
     A[q] = killed ? 0.0 : PK[q] - beta * ((q % 4) == 0 ? F[q] - 1.0 : F[q]);
@@ -138,7 +157,7 @@ __device__ __forceinline__ bool c_point64(const DevBody& d, const DevParam& P, l
                                           unsigned meta, int cnt, int na, const double* K,
                                           const double* Ft) {
   const double damage = 1.0 - (double)na / (double)cnt;
-  double Kinv[9], F[9], PKinv[9];
+  double Kinv[9], F[9], PKinv[9], C1[9];
   inv3(K, Kinv);
   matmul3(Ft, Kinv, F);
   bool hasnan = false;
@@ -153,12 +172,11 @@ __device__ __forceinline__ bool c_point64(const DevBody& d, const DevParam& P, l
     matmul3(Pm, Kinv, PKinv);
     for (int q = 0; q < 9; q++) d.PK64[9 * i + q] = PKinv[q];
     if (d.zem == ZEM_WAN) {
-      double C1[9];
       zem_wan64(P, Kinv, C1);
       for (int q = 0; q < 9; q++) d.C164[9 * i + q] = C1[q];
     }
   }
-  c_state64(d, i, killed, P.beta, F, PKinv);
+  c_state64(d, i, killed, P.beta, F, PKinv, C1);
   d.n_active[i] = na;
   return killed;
 }
