@@ -62,6 +62,13 @@ static void destroy_graph(pd_handle* h) {
   h->gkey = GraphKey();
 }
 
+// what a captured step holds (bond arrays, bond-state mode, parameters) changed: the handle's graph
+// goes, and the graphs of the groups that the handle belongs to no longer match its version
+static void drop_graphs(pd_handle* h) {
+  destroy_graph(h);
+  h->version++;
+}
+
 extern "C" const char* pd_last_error(void) { return g_err.c_str(); }
 extern "C" const char* pd_version(void) { return "0.1.0"; }
 
@@ -159,7 +166,6 @@ static pd_status ensure_tiles(pd_handle* h) {
   h->d.lidx = t.lidx;
   h->d.lown = t.lown;
   h->d.tile_cap = t.cap;
-  h->version++;
   if (h->precision == PD_PREC_FP64) return PD_OK;
   unsigned* cls = nullptr;
   float4* geo = nullptr;
@@ -389,7 +395,7 @@ static pd_status relayout(pd_handle* h, int G) {
   h->tiles_tried = false;
   h->d = b;
   h->nslots = nslots;
-  destroy_graph(h);
+  drop_graphs(h);
   return ensure_tiles(h);
 }
 
@@ -812,7 +818,7 @@ extern "C" pd_status pd_set_state(pd_handle* h, const double* position, const do
     launch_count_active(h->d, h->stream);
     h->damage_valid = true;
     PD_TRY(check_symmetry(h));
-    destroy_graph(h);
+    drop_graphs(h);
   }
   PD_TRY(clear_error(h));
   PD_CUDA(cudaStreamSynchronize(h->stream));
@@ -1002,8 +1008,7 @@ extern "C" pd_status pd_set_bcs(pd_handle* h, int32_t n_bcs, const pd_bc_desc* b
   const long long zero = 0;
   PD_TRY(set_ctrl(h, offsetof(Ctrl, table_n), &zero, sizeof(long long)));
   PD_CUDA(cudaStreamSynchronize(h->stream));
-  h->version++;
-  destroy_graph(h);
+  drop_graphs(h);
   return PD_OK;
 }
 
@@ -1064,7 +1069,7 @@ extern "C" pd_status pd_set_param_timesteps(pd_handle* h, const double* dtp) {
   PD_CUDA(cudaSetDevice(h->device));
   for (size_t k = 0; k < h->hp.size(); k++) { h->hp[k].dt = dtp[k]; h->hp[k].dth = 0.5 * dtp[k]; }
   PD_TRY(upload_params(h));
-  destroy_graph(h);
+  drop_graphs(h);
   return PD_OK;
 }
 
@@ -1453,7 +1458,7 @@ extern "C" pd_status pd_set_mapping(pd_handle* h, int32_t group, int32_t block) 
     if (group != 1) h->cfg.pipe = 0;
   }
   h->cfg.block = block;
-  destroy_graph(h);
+  drop_graphs(h);
   return PD_OK;
 }
 
@@ -1525,7 +1530,7 @@ extern "C" pd_status pd_autotune(pd_handle* h, int32_t* group_out, int32_t* bloc
     if (c.ms < best) { best = c.ms; bestc = c.c; }
   PD_TRY(relayout(h, bestc.group));
   h->cfg = bestc;
-  destroy_graph(h);
+  drop_graphs(h);
   if (group_out) *group_out = bestc.group;
   if (block_out) *block_out = bestc.block;
   return check_err(h);
@@ -1535,7 +1540,7 @@ extern "C" pd_status pd_set_graph(pd_handle* h, int32_t steps_per_graph) {
   if (!h) return fail(PD_ERR_ARG, "handle is NULL");
   if (steps_per_graph < 0 || steps_per_graph > 4096) return fail(PD_ERR_ARG, "0 <= steps_per_graph <= 4096");
   h->graph_steps = steps_per_graph;
-  destroy_graph(h);
+  drop_graphs(h);
   return PD_OK;
 }
 
@@ -1579,7 +1584,7 @@ extern "C" pd_status pd_break_bonds(pd_handle* h, const uint8_t* set_a, const ui
   cudaFree(tmp);
   if (e != cudaSuccess) return fail(PD_ERR_CUDA, cudaGetErrorString(e));
   h->damage_valid = true;
-  destroy_graph(h);
+  drop_graphs(h);
   return PD_OK;
 }
 
@@ -1627,7 +1632,7 @@ extern "C" pd_status pd_break_random_pairs_ids(pd_handle* h, double fraction, ui
   dfree(h, gid);
   h->damage_valid = true;
   PD_TRY(check_symmetry(h));
-  destroy_graph(h);
+  drop_graphs(h);
   return PD_OK;
 }
 
@@ -1649,7 +1654,7 @@ extern "C" pd_status pd_set_pipeline(pd_handle* h, int32_t pipe) {
   if (pipe >= 1 && pipe <= 3 && (h->precision != PD_PREC_FP32_KAHAN || !tma_supported(h->d)))
     return fail(PD_ERR_ARG, "the staged bond stream needs the FP32 path, one lane per point and BB or OSB");
   h->cfg.pipe = pipe;
-  destroy_graph(h);
+  drop_graphs(h);
   return PD_OK;
 }
 
