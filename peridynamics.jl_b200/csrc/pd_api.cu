@@ -1147,7 +1147,9 @@ static pd_status run_block_graph(pd_handle* h, int steps, double dto) {
     long long before = h->launches;
     PD_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     issue_steps(h, steps, dto, nullptr);
+    const cudaError_t le = cudaGetLastError();  // a launch that was refused
     cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
+    if (e == cudaSuccess && le != cudaSuccess) { cudaGraphDestroy(graph); e = le; }
     if (e != cudaSuccess) return fail(PD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
     h->graph_nodes = (int)(h->launches - before);
     h->launches = before;
@@ -1335,7 +1337,9 @@ extern "C" pd_status pd_group_run_vv(pd_group* g, int64_t first_step, int64_t n_
         cudaError_t e = cudaStreamBeginCapture(origin, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
           group_issue(g, steps, dto);
+          const cudaError_t le = cudaGetLastError();  // a launch that was refused
           e = cudaStreamEndCapture(origin, &graph);
+          if (e == cudaSuccess && le != cudaSuccess) { cudaGraphDestroy(graph); e = le; }
         }
         g->nodes.assign(g->hs.size(), 0);
         for (size_t k = 0; k < g->hs.size(); k++) {

@@ -96,6 +96,15 @@ void launch_split_u_rows(const DevBody& d, const int* rows, long long n, cudaStr
 // arrays are the caller's to free; a body with a tile of more than TILE_MAX points has no tiles
 // (pt null)
 constexpr int TILE_MAX = 4095;  // 16-byte records that a 16-bit byte offset reaches
+// Dynamic shared memory of a tile kernel at most: the 227 KB of a block less 8 KB for its segment sums.
+// The limit of a kernel belongs to the context, not to a body: every launch sets this one, so that no
+// host thread lowers it between another's setting and launch. A failure is the last CUDA error, which the
+// callers read.
+constexpr int TILE_SMEM = 219 * 1024;
+template <class K>
+inline bool allow_tile_smem(K kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM) == cudaSuccess;
+}
 struct PlaceGrid {
   double lo[3], inv;
   int axis[3];

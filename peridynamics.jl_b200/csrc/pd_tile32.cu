@@ -531,7 +531,7 @@ static int state_bytes(const DevBody& d, int phase) {
 
 // a tile, its classes and the segment sums of the warps that share a slice fit the 227 KB of a block
 bool tile32_supported(const DevBody& d, int phase) {
-  return d.tile_pt != nullptr && tile_bytes(d.tile_cap, state_bytes(d, phase), d.ncls) + 8 * 1024 <= 227 * 1024;
+  return d.tile_pt != nullptr && tile_bytes(d.tile_cap, state_bytes(d, phase), d.ncls) <= TILE_SMEM;
 }
 
 // Warps per slice: the largest of 8, 4, 2, 1 that keeps the launch within the 24 warps per SM that
@@ -545,11 +545,9 @@ static int tile_split(const DevBody& d) {
   return W;
 }
 
-// The attribute belongs to the current device's context: set on every launch.
 #define PD_TILE_LAUNCH(W, K)                                                               \
   do {                                                                                     \
-    cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);            \
-    K<<<grid * (W), 32 * TILE_SLICES, smem, s>>>(d, kstep);                                \
+    if (allow_tile_smem(K)) K<<<grid * (W), 32 * TILE_SLICES, smem, s>>>(d, kstep);        \
   } while (0)
 #define PD_TILE_W(CALL)                                            \
   switch (W) {                                                     \

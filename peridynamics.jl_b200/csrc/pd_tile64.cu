@@ -324,13 +324,12 @@ static int split64(const DevBody& d) {
 bool tile64_supported(const DevBody& d, int phase) {
   if (d.tile_pt == nullptr || d.len64 == nullptr || d.material == MAT_CMAT || d.multi || d.sc64) return false;
   if (phase == 2 && (!d.sym || split64(d) > 1)) return false;
-  return tile_bytes64(d, phase) + 8 * 1024 <= 227 * 1024;  // and the segment sums
+  return tile_bytes64(d, phase) <= TILE_SMEM;
 }
 
 #define PD_TILE_LAUNCH64(W, K)                                                             \
   do {                                                                                     \
-    cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);            \
-    K<<<grid * (W), 32 * TILE_SLICES, smem, s>>>(d, kstep);                                \
+    if (allow_tile_smem(K)) K<<<grid * (W), 32 * TILE_SLICES, smem, s>>>(d, kstep);        \
   } while (0)
 #define PD_TILE_W64(CALL)                                          \
   switch (W) {                                                     \
