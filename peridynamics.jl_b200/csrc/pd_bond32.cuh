@@ -129,18 +129,27 @@ __device__ __forceinline__ float2 osb_point(const DevParam& P, float w, float t,
   return make_float2((float)(15.0 * P.G * rw), (float)(th * (3.0 * P.K - 5.0 * P.G) * rw));
 }
 
-// the force on a point: its sum times the factor f that all bonds share (in double, as above)
+// the force on a point: its sum times the factor f that all bonds share (in double, as above). A point
+// without a bond has none, wherever it is: at infinity its own bond vectors (0 times them is added) are
+// undefined
 __device__ __forceinline__ void store_force(const DevBody& d, long long i, int kstep, double f,
                                             const float2 v, float vz) {
-  const float x = (float)(f * (double)v.x), y = (float)(f * (double)v.y), z = (float)(f * (double)vz);
+  float x = (float)(f * (double)v.x), y = (float)(f * (double)v.y), z = (float)(f * (double)vz);
+  if (isnan(x) || isnan(y) || isnan(z)) {
+    bool bonded = false;
+    const int cnt = (int)(d.off[i + 1] - d.off[i]);
+    for (int k = 0; k < cnt && !bonded; k++) bonded = bond_bit_live(d.bits, bond_slot(d, i, k));
+    if (bonded) {
+      const long long step = d.ctrl->base + kstep;
+      if (atomicExch(&d.ctrl->err, 1) == 0) d.ctrl->err_step = step;
+      else atomicMin(&d.ctrl->err_step, step);
+    } else {
+      x = y = z = 0.f;
+    }
+  }
   d.b32[3 * i] = x;
   d.b32[3 * i + 1] = y;
   d.b32[3 * i + 2] = z;
-  if (isnan(x) || isnan(y) || isnan(z)) {
-    const long long step = d.ctrl->base + kstep;
-    if (atomicExch(&d.ctrl->err, 1) == 0) d.ctrl->err_step = step;
-    else atomicMin(&d.ctrl->err_step, step);
-  }
 }
 
 // correspondence phase A: the constants of a point

@@ -138,8 +138,20 @@ struct TileStream {
   }
 };
 
+// A broken bond adds zero times its vector, and a neighbour that a point has lost may be anywhere, at
+// infinity too. NEAR: the tile holds every displacement within +-1e37 and its low part within +-1e30 (below
+// 2^-24 of that), where zero times a bond vector is zero and an unbroken bond to such a point still has no
+// defined length. A select of the point itself in the loop costs the BB kernel registers that it spills
+// (17.8 -> 18.9 ms for 40 steps of 1M points); correspondence, which spills none and multiplies the
+// displacement by the stabilising stiffness, takes the select.
+constexpr float FAR32 = 1e37f, FAR32_LO = 1e30f;
+__device__ __forceinline__ float4 near32(const float4& u, float far) {
+  return make_float4(fminf(fmaxf(u.x, -far), far), fminf(fmaxf(u.y, -far), far),
+                     fminf(fmaxf(u.z, -far), far), u.w);
+}
+
 // one block: its tile in shared memory, the place of every thread
-template <bool CLS, int NS, int W>
+template <bool CLS, int NS, int W, bool NEAR>
 struct Tile {
   char* sm;
   unsigned c16;          // bytes of one array of 16-byte records
@@ -161,8 +173,9 @@ struct Tile {
 #pragma unroll 4
     for (int k = threadIdx.x; k < n; k += 32 * TILE_SLICES) {
       const int p = __ldg(list + k);
-      *reinterpret_cast<float4*>(sm + 16 * k) = __ldg(d.uhi + p);
-      *reinterpret_cast<float4*>(sm + c16 + 16 * k) = __ldg(d.ulo + p);
+      const float4 h = __ldg(d.uhi + p), l = __ldg(d.ulo + p);
+      *reinterpret_cast<float4*>(sm + 16 * k) = NEAR ? near32(h, FAR32) : h;
+      *reinterpret_cast<float4*>(sm + c16 + 16 * k) = NEAR ? near32(l, FAR32_LO) : l;
       if constexpr (NS == 8)
         *reinterpret_cast<float2*>(sm + 2 * c16 + 8 * k) = __ldg(d.cc32 + p);
       if constexpr (NS == 40) {
@@ -263,6 +276,12 @@ __device__ __forceinline__ ACC walk_rows(ST& st, int rows, int part, int lane, F
   return tot;
 }
 
+// Whether the tile has the point at the end of its range: two such points are not at rest. (OSB has seen
+// that in phase A.)
+__device__ __forceinline__ bool far_off(const Own32& o) {
+  return !(fmaxf(fmaxf(fabsf(o.nhi.x), fabsf(o.nhi.y)), fabsf(o.nhz)) < FAR32);
+}
+
 // a force sum and a count
 struct ForceSum {
   KSum2 xy;
@@ -315,7 +334,7 @@ extern __shared__ __align__(16) char tile_smem[];
 // BB (bond_based.jl:125-161)
 template <bool CLS, int W>
 __global__ void __launch_bounds__(256, MT_BB) k_bb32s(DevBody d, int kstep) {
-  Tile<CLS, 0, W> t;
+  Tile<CLS, 0, W, true> t;
   if (!t.begin(d, tile_smem)) return;
   const DevParam& P = d.params[t.valid ? d.meta[t.i] & META_PID_MASK : 0];
   const float epsc = P.epscf;
@@ -340,7 +359,7 @@ __global__ void __launch_bounds__(256, MT_BB) k_bb32s(DevBody d, int kstep) {
   });
   if (t.valid && t.part == 0) {
     if (S.lost) d.n_active[t.i] -= S.lost;
-    store_force(d, t.i, kstep, P.bc, S.xy.value(), S.z.value());
+    store_force(d, t.i, kstep, P.bc, S.xy.value(), far_off(own) ? NAN : S.z.value());
   }
 }
 
@@ -348,7 +367,7 @@ __global__ void __launch_bounds__(256, MT_BB) k_bb32s(DevBody d, int kstep) {
 // the bonds that break (FULLM: summed in full), dilatation, c1 and c2
 template <bool CLS, int W, bool FULLM, bool LIN>
 __global__ void __launch_bounds__(256, MT_A) k_osb_a32s(DevBody d, int kstep) {
-  Tile<CLS, 0, W> t;
+  Tile<CLS, 0, W, false> t;
   if (!t.begin(d, tile_smem)) return;
   const DevParam& P = d.params[t.valid ? d.meta[t.i] & META_PID_MASK : 0];
   const float epsc = P.epscf;
@@ -408,7 +427,7 @@ __global__ void __launch_bounds__(256, MT_A) k_osb_a32s(DevBody d, int kstep) {
 // OSB phase B (ordinary_state_based.jl:128-174) for symmetric bond states
 template <bool CLS, int W, bool LIN>
 __global__ void __launch_bounds__(256, MT_B) k_osb_b32s(DevBody d, int kstep) {
-  Tile<CLS, 8, W> t;
+  Tile<CLS, 8, W, true> t;
   if (!t.begin(d, tile_smem)) return;
   const DevParam& P = d.params[t.valid ? d.meta[t.i] & META_PID_MASK : 0];
   const Influence om(d, P);
@@ -439,7 +458,7 @@ struct CorrAcc : CorrSums<FULLK> {
 // CMat phase A (correspondence.jl:193-224, 288-298; bond_system.jl:309-327)
 template <bool CLS, bool FULLK, bool LIN>
 __global__ void __launch_bounds__(256, MT_CA) k_c_a32s(DevBody d, int kstep) {
-  Tile<CLS, 0, 1> t;
+  Tile<CLS, 0, 1, false> t;
   if (!t.begin(d, tile_smem)) return;
   const unsigned meta = t.valid ? d.meta[t.i] : 0u;
   const DevParam& P = d.params[meta & META_PID_MASK];
@@ -451,10 +470,11 @@ __global__ void __launch_bounds__(256, MT_CA) k_c_a32s(DevBody d, int kstep) {
     bool act[2];
 #pragma unroll
     for (int u = 0; u < 2; u++) {
-      const float4 hj = t.hi(p.key[u]);
+      const unsigned k = p.a[u] ? p.key[u] : t.own;
+      const float4 hj = t.hi(k);
       float2 dxy;
       float dz, num;
-      bond_du(p.g[u], hj, t.lo(p.key[u]), own, dxy, dz, num);
+      bond_du(p.g[u], hj, t.lo(k), own, dxy, dz, num);
       const float rL = st.rL(p, u);
       act[u] = corr_stays(p.a[u], cp, p.g[u], rL, dxy, dz, num);
       const float w = corr_weight<LIN>(cp, p.g[u], rL, hj.w);
@@ -501,7 +521,7 @@ __global__ void __launch_bounds__(256, MT_CA) k_c_a32s(DevBody d, int kstep) {
 // CMat phase B (correspondence.jl:226-251) for ZEMSilling and symmetric bond states
 template <bool CLS, int W, bool LIN>
 __global__ void __launch_bounds__(256, MT_CB) k_c_b32s(DevBody d, int kstep) {
-  Tile<CLS, 40, W> t;
+  Tile<CLS, 40, W, false> t;
   if (!t.begin(d, tile_smem)) return;
   const DevParam& P = d.params[t.valid ? d.meta[t.i] & META_PID_MASK : 0];
   const Influence om(d, P);
@@ -512,11 +532,12 @@ __global__ void __launch_bounds__(256, MT_CB) k_c_b32s(DevBody d, int kstep) {
   const ForceSum S = walk_rows<W, ForceSum>(st, t.rows, t.part, t.lane, [&](const Pair32& p, int r, ForceSum& s) {
 #pragma unroll
     for (int u = 0; u < 2; u++) {
-      const float4 hj = t.hi(p.key[u]);
+      const unsigned k = p.a[u] ? p.key[u] : t.own;
+      const float4 hj = t.hi(k);
       float2 dxy, txy;
       float dz, num, tz;
-      bond_du(p.g[u], hj, t.lo(p.key[u]), own, dxy, dz, num);
-      corr_pair(p.g[u], dxy, dz, ia, ib, ic, t.sa(p.key[u]), t.sb(p.key[u]), t.sc(p.key[u]), txy, tz);
+      bond_du(p.g[u], hj, t.lo(k), own, dxy, dz, num);
+      corr_pair(p.g[u], dxy, dz, ia, ib, ic, t.sa(k), t.sb(k), t.sc(k), txy, tz);
       const float f = (LIN ? st.rL(p, u) : om.at<LIN>(fabsf(p.g[u].w), 0.f)) * hj.w;
       s.add(p.a[u] ? f : 0.f, txy, tz);
     }
