@@ -15,6 +15,7 @@
 // CSR bond arrays instead of the sliced layout.
 #include <cuda.h>
 
+#include <cfloat>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -123,7 +124,8 @@ __global__ void __launch_bounds__(256) k_static_osb_a(StaticArgs a) {
     s_diff(a.x, xi, j, d);
     s_diff(a.X, Xi, j, D);
     const double l2 = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2];
-    const double e = sqrt_of(l2, rsqrt3(l2)) - L;
+    // two points in one place: no reciprocal of the length, but a dilatation
+    const double e = l2 < DBL_MIN ? -L : sqrt_of(l2, rsqrt3(l2)) - L;
     if (!(L > 0 && e < thr * L) && (sqrt(l2) - L) / L > a.epsc && a.fail_permit[b]) {
       a.bond_active[b] = 0;
       act = 0;
