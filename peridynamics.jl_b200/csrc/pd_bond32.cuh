@@ -120,11 +120,11 @@ __device__ __forceinline__ float osb_pair(const Influence& om, const BondP& B, f
 // dilatation's terms. In double: a factor rounded here moves all of the point's bonds the same way
 // (relative error of the forces against 64 bits, 975-point coupon: 9.2e-8 in float, 8.0e-8 so).
 template <bool LIN>
-__device__ __forceinline__ float2 osb_point(const DevParam& P, float w, float t, float& dil) {
+__device__ __forceinline__ float2 osb_point(const DevParam& P, float w, double t, float& dil) {
   dil = 0.f;
   if (w == 0.f) return make_float2(0.f, 0.f);
   const double rw = 1.0 / (double)w;
-  const double th = 3.0 * rw * (LIN ? P.delta * (double)t : (double)t);
+  const double th = 3.0 * rw * (LIN ? P.delta * t : t);
   dil = (float)th;
   return make_float2((float)(15.0 * P.G * rw), (float)(th * (3.0 * P.K - 5.0 * P.G) * rw));
 }
@@ -133,8 +133,9 @@ __device__ __forceinline__ float2 osb_point(const DevParam& P, float w, float t,
 // without a bond has none, wherever it is: at infinity its own bond vectors (0 times them is added) are
 // undefined
 __device__ __forceinline__ void store_force(const DevBody& d, long long i, int kstep, double f,
-                                            const float2 v, float vz) {
-  float x = (float)(f * (double)v.x), y = (float)(f * (double)v.y), z = (float)(f * (double)vz);
+                                            const KSum2& xy, const KSum1& zs) {
+  float x = (float)(f * ((double)xy.s.x + (double)xy.n.x)), y = (float)(f * ((double)xy.s.y + (double)xy.n.y)),
+        z = (float)(f * ((double)zs.s + (double)zs.n));
   if (isnan(x) || isnan(y) || isnan(z)) {
     bool bonded = false;
     const int cnt = (int)(d.off[i + 1] - d.off[i]);

@@ -962,7 +962,7 @@ __global__ void __launch_bounds__(256, PD_MINB_CQB) k_c_b32q(DevBody d, int kste
     }
     if (valid) {
       // the linear influence function is delta / L: delta leaves the sums
-      store_force(d, i, kstep, LIN ? P.delta : 1.0, sxy.value(), sz.value());
+      store_force(d, i, kstep, LIN ? P.delta : 1.0, sxy, sz);
     }
   }
 }

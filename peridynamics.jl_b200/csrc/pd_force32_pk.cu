@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256, PD_MINB_QB) k_osb_b32q(DevBody d, int kst
       }
     }
     if (valid) {
-      store_force(d, i, kstep, LIN ? P.delta : 1.0, txy.value(), tz.value());
+      store_force(d, i, kstep, LIN ? P.delta : 1.0, txy, tz);
     }
   }
 }
@@ -209,15 +209,15 @@ __global__ void __launch_bounds__(256, PD_MINB_QA) k_osb_a32q(DevBody d, int kst
       }
     }
     if (valid) {
-      float wv, tv;
+      float wv;
+      double tv;
       if (FULLM) {
-        const float2 v = tmt.value();
-        wv = v.x;
-        tv = v.y;
+        wv = tmt.value().x;
+        tv = (double)tmt.s.y + (double)tmt.n.y;
       } else {
         const float m0 = d.cm32[i].x;
         wv = tdm != 0.f ? m0 - tdm : m0;
-        tv = tth.value();
+        tv = (double)tth.s + (double)tth.n;
       }
       float dil;
       d.cc32[i] = osb_point<LIN>(P, wv, tv, dil);
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(256, PD_MINB_QBB) k_bb32q(DevBody d, int kstep
     }
     if (valid) {
       d.n_active[i] = na;
-      store_force(d, i, kstep, P.bc, txy.value(), tz.value());
+      store_force(d, i, kstep, P.bc, txy, tz);
     }
   }
 }

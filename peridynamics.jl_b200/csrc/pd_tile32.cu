@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(256, MT_BB) k_bb32s(DevBody d, int kstep) {
   const float epsc = P.epscf;
   const Own32 own(t.hi(t.own), t.lo(t.own));
   TileStream<CLS, true> st(d, t.geo, t.rl, t.sbase, t.rows, t.lane);
-  const ForceSum S = walk_rows<W, ForceSum>(st, t.rows, t.part, t.lane, [&](const Pair32& p, int r, ForceSum& s) {
+  ForceSum S = walk_rows<W, ForceSum>(st, t.rows, t.part, t.lane, [&](const Pair32& p, int r, ForceSum& s) {
     bool act[2];
 #pragma unroll
     for (int u = 0; u < 2; u++) {
@@ -358,8 +358,9 @@ __global__ void __launch_bounds__(256, MT_BB) k_bb32s(DevBody d, int kstep) {
     }
   });
   if (t.valid && t.part == 0) {
+    if (far_off(own)) S.z.s = NAN;
     if (S.lost) d.n_active[t.i] -= S.lost;
-    store_force(d, t.i, kstep, P.bc, S.xy.value(), far_off(own) ? NAN : S.z.value());
+    store_force(d, t.i, kstep, P.bc, S.xy, S.z);
   }
 }
 
@@ -406,15 +407,15 @@ __global__ void __launch_bounds__(256, MT_A) k_osb_a32s(DevBody d, int kstep) {
     }
   });
   if (t.valid && t.part == 0) {
-    float wv, tv;
+    float wv;
+    double tv;
     if constexpr (FULLM) {
-      const float2 v = S.mt.value();
-      wv = v.x;
-      tv = v.y;
+      wv = S.mt.value().x;
+      tv = (double)S.mt.s.y + (double)S.mt.n.y;
     } else {
       const float m0 = d.cm32[t.i].x;
       wv = S.dm != 0.f ? m0 - S.dm : m0;
-      tv = S.th.value();
+      tv = (double)S.th.s + (double)S.th.n;
     }
     float dil;
     d.cc32[t.i] = osb_point<LIN>(P, wv, tv, dil);
@@ -445,7 +446,7 @@ __global__ void __launch_bounds__(256, MT_B) k_osb_b32s(DevBody d, int kstep) {
     }
   });
   if (t.valid && t.part == 0)
-    store_force(d, t.i, kstep, LIN ? P.delta : 1.0, S.xy.value(), S.z.value());
+    store_force(d, t.i, kstep, LIN ? P.delta : 1.0, S.xy, S.z);
 }
 
 // the sums of correspondence phase A and its count; not cut into segments (their sums would take
@@ -543,7 +544,7 @@ __global__ void __launch_bounds__(256, MT_CB) k_c_b32s(DevBody d, int kstep) {
     }
   });
   if (t.valid && t.part == 0)
-    store_force(d, t.i, kstep, LIN ? P.delta : 1.0, S.xy.value(), S.z.value());
+    store_force(d, t.i, kstep, LIN ? P.delta : 1.0, S.xy, S.z);
 }
 
 static int state_bytes(const DevBody& d, int phase) {
