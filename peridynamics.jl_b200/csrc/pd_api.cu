@@ -85,6 +85,7 @@ static DevParam make_param(const pd_point_params& p, double cs) {
   q.zwaf = (float)q.zwa;
   q.inv_delta = (float)(1.0 / p.delta);
   q.vscale = (float)(1.0 / (p.delta * p.delta * p.delta));
+  q.wratio = (double)q.deltaf / p.delta;
   return q;
 }
 

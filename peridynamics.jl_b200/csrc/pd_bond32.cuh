@@ -123,7 +123,7 @@ template <bool LIN>
 __device__ __forceinline__ float2 osb_point(const DevParam& P, float w, double t, float& dil) {
   dil = 0.f;
   if (w == 0.f) return make_float2(0.f, 0.f);
-  const double rw = 1.0 / (double)w;
+  const double rw = (LIN ? P.wratio : 1.0) / (double)w;
   const double th = 3.0 * rw * (LIN ? P.delta * t : t);
   dil = (float)th;
   return make_float2((float)(15.0 * P.G * rw), (float)(th * (3.0 * P.K - 5.0 * P.G) * rw));

@@ -68,6 +68,10 @@ struct DevParam {
   float deltaf, bcf, epscf, Gf, Kf, lambdaf, muf, betaf, zwaf;
   float inv_delta;  // 1 / delta (FP32 correspondence scaling)
   float vscale;     // 1 / delta^3 (FP32 correspondence scaling)
+  // (float)delta / delta: the packed FP32 OSB kernels take the linear influence function's factor delta
+  // out of the sums of forces and dilatations and apply it in double, but sum the weighted volume with
+  // (float)delta; the quotient belongs to the inverse weighted volume, else it moves all forces of a body
+  double wratio;
 };
 
 struct Ctrl {
