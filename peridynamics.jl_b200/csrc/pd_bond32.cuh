@@ -183,27 +183,43 @@ __device__ __forceinline__ float corr_weight(const CorrA& c, const float4& g, fl
   return (LIN ? rL : c.om.at<LIN>(fabsf(g.w), rL)) * V * c.ks;
 }
 
-// the sums of correspondence phase A: the displacement gradient (rows x, y of every column packed;
-// plain FP32 sums: compensated ones moved the displacement after 250 steps by less than the error
-// of the form) and, in full, the shape tensor {xx, yy, zz, xy, xz, yz} (compensated)
-template <bool FULLK>
+// The sums of correspondence phase A: the displacement gradient (rows x, y of every column packed) and, in
+// full, the shape tensor {xx, yy, zz, xy, xz, yz} (compensated). COMP: compensated sums of the gradient, else
+// plain FP32 ones, which bond-stream variant 5 asks for (their error in the displacement after 250 steps is
+// less than the rest of the form's)
+template <bool FULLK, bool COMP>
 struct CorrSums {
-  float2 Hxy[3];
-  float Hz[3];
+  static constexpr bool FULL = FULLK;
+  float2 Hxy[3], nxy[3];  // COMP: the sums and their negated compensations
+  float Hz[3], nz[3];
   KSum2 K01, K23, K45;
   float dK[6];
   __device__ __forceinline__ CorrSums() {
 #pragma unroll
-    for (int c = 0; c < 3; c++) { Hxy[c] = both(0.f); Hz[c] = 0.f; }
+    for (int c = 0; c < 3; c++) { Hxy[c] = nxy[c] = both(0.f); Hz[c] = nz[c] = 0.f; }
 #pragma unroll
     for (int q = 0; q < 6; q++) dK[q] = 0.f;
+  }
+  // column c gains f times du
+  __device__ __forceinline__ void column(int c, float f, const float2 dxy, float dz) {
+    if constexpr (COMP) {
+      const float2 y = fma2(both(f), dxy, nxy[c]), t = add2(Hxy[c], y);
+      nxy[c] = add2(sub2(Hxy[c], t), y);
+      Hxy[c] = t;
+      const float yz = fmaf(f, dz, nz[c]), tz = Hz[c] + yz;
+      nz[c] = (Hz[c] - tz) + yz;
+      Hz[c] = tz;
+    } else {
+      Hxy[c] = fma2(both(f), dxy, Hxy[c]);
+      Hz[c] = fmaf(f, dz, Hz[c]);
+    }
   }
   __device__ __forceinline__ void add(float t, const float4& g, const float2 dxy, float dz) {
     const float2 tX = mul2(both(t), xy(g));
     const float tXz = t * g.z;
-    Hxy[0] = fma2(both(tX.x), dxy, Hxy[0]); Hz[0] = fmaf(tX.x, dz, Hz[0]);
-    Hxy[1] = fma2(both(tX.y), dxy, Hxy[1]); Hz[1] = fmaf(tX.y, dz, Hz[1]);
-    Hxy[2] = fma2(both(tXz), dxy, Hxy[2]);  Hz[2] = fmaf(tXz, dz, Hz[2]);
+    column(0, tX.x, dxy, dz);
+    column(1, tX.y, dxy, dz);
+    column(2, tXz, dxy, dz);
     if constexpr (FULLK) {
       K01.add(mul2(tX, xy(g)));
       K23.add(make_float2(tXz * g.z, tX.x * g.y));

@@ -829,7 +829,7 @@ __global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kste
     const int* pn = d.nbr + sbase + lane;
     const float4* pg = d.geo + sbase + lane;
     unsigned* pw = d.bits + (sbase >> 5);
-    CorrSums<FULLK> S;
+    CorrSums<FULLK, false> S;
     int na = 0;
     int nj0 = self, nj1 = self;
     float4 ng0 = make_float4(0.f, 0.f, 0.f, 1.f), ng1 = ng0;
@@ -877,7 +877,7 @@ __global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kste
         if (two && c1 != w1) pw[r + 1] = c1;
       }
     }
-    const bool killed = valid && corr_point32<FULLK>(d, P, i, meta, cnt, na, S);
+    const bool killed = valid && corr_point32(d, P, i, meta, cnt, na, S);
     if (!d.sym) {
       // directed bond states: a killed point loses all its bonds (correspondence.jl:293)
       const unsigned kill_mask = __ballot_sync(0xffffffffu, killed);

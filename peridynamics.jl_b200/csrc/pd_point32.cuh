@@ -128,14 +128,13 @@ __device__ __forceinline__ void c_state_clear32(const DevBody& d, long long i) {
 
 // From the sums of a point: F - I, the kill decision (too_much_damage!, correspondence.jl:288-298)
 // and the phase-B state. Returns whether the point is killed.
-template <bool FULLK>
+template <class SUMS>
 __device__ __forceinline__ bool corr_point32(const DevBody& d, const DevParam& P, long long i,
-                                             unsigned meta, int cnt, int na,
-                                             const pack::CorrSums<FULLK>& S) {
+                                             unsigned meta, int cnt, int na, const SUMS& S) {
   const float id = P.inv_delta;
   float k6[6];
   float2* ks = reinterpret_cast<float2*>(d.K32 + 6 * i);
-  if constexpr (FULLK) {
+  if constexpr (SUMS::FULL) {
     const float2 v01 = S.K01.value(), v23 = S.K23.value(), v45 = S.K45.value();
     k6[0] = v01.x; k6[1] = v01.y; k6[2] = v23.x; k6[3] = v23.y; k6[4] = v45.x; k6[5] = v45.y;
     ks[0] = make_float2(k6[0], k6[1]); ks[1] = make_float2(k6[2], k6[3]); ks[2] = make_float2(k6[4], k6[5]);
@@ -155,7 +154,9 @@ __device__ __forceinline__ bool corr_point32(const DevBody& d, const DevParam& P
   finv3(Km, Kinv);
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    Hm[3 * c] = S.Hxy[c].x; Hm[3 * c + 1] = S.Hxy[c].y; Hm[3 * c + 2] = S.Hz[c];
+    Hm[3 * c] = S.Hxy[c].x + S.nxy[c].x;
+    Hm[3 * c + 1] = S.Hxy[c].y + S.nxy[c].y;
+    Hm[3 * c + 2] = S.Hz[c] + S.nz[c];
   }
   fmatmul(Hm, Kinv, H);
   bool hasnan = false;

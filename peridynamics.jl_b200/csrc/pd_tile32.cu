@@ -323,9 +323,9 @@ struct DilSum<true> {
 
 // Resident blocks of 256 threads per SM, measured on 1M-point blocks (us a launch): BB 4 blocks (64
 // registers) 295 / 3 361 / 5 426; OSB phase A 4 blocks 287 / 3 360 / 5 406, full geometry stream 438 /
-// 476 / 701; OSB phase B 3 blocks (80 registers) 336 / 4 377; CMat phase A 3 blocks 403 / 2 507, phase
-// B 2 blocks (tiles of 72 bytes a point fill the SM) 537 / 3 579.
-constexpr int MT_BB = 4, MT_A = 4, MT_B = 3, MT_CA = 3, MT_CB = 2;
+// 476 / 701; OSB phase B 3 blocks (80 registers) 336 / 4 377; CMat phase A 3 blocks 403 / 2 507, with
+// compensated sums 2 blocks 525, phase B 2 blocks (tiles of 72 bytes a point fill the SM) 537 / 3 579.
+constexpr int MT_BB = 4, MT_A = 4, MT_B = 3, MT_CA = 3, MT_CAK = 2, MT_CB = 2;
 
 }  // namespace
 
@@ -451,21 +451,21 @@ __global__ void __launch_bounds__(256, MT_B) k_osb_b32s(DevBody d, int kstep) {
 
 // the sums of correspondence phase A and its count; not cut into segments (their sums would take
 // their registers twice), so always one warp a slice
-template <bool FULLK>
-struct CorrAcc : CorrSums<FULLK> {
+template <bool FULLK, bool COMP>
+struct CorrAcc : CorrSums<FULLK, COMP> {
   int na = 0;  // FULLK: the active bonds; else the bonds that break in this evaluation
 };
 
 // CMat phase A (correspondence.jl:193-224, 288-298; bond_system.jl:309-327)
-template <bool CLS, bool FULLK, bool LIN>
-__global__ void __launch_bounds__(256, MT_CA) k_c_a32s(DevBody d, int kstep) {
+template <bool CLS, bool FULLK, bool LIN, bool COMP>
+__global__ void __launch_bounds__(256, COMP ? MT_CAK : MT_CA) k_c_a32s(DevBody d, int kstep) {
   Tile<CLS, 0, 1, false> t;
   if (!t.begin(d, tile_smem)) return;
   const unsigned meta = t.valid ? d.meta[t.i] : 0u;
   const DevParam& P = d.params[meta & META_PID_MASK];
   const CorrA cp(d, P);
   const Own32 own(t.hi(t.own), t.lo(t.own));
-  CorrAcc<FULLK> S;
+  CorrAcc<FULLK, COMP> S;
   TileStream<CLS, true> st(d, t.geo, t.rl, t.sbase, t.rows, t.lane);
   auto pair = [&](const Pair32& p, int r) {
     bool act[2];
@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(256, MT_CA) k_c_a32s(DevBody d, int kstep) {
   if (t.valid) {
     const int cnt = (int)(d.off[t.i + 1] - d.off[t.i]);
     const int na = FULLK ? S.na : d.n_active[t.i] - S.na;
-    killed = corr_point32<FULLK>(d, P, t.i, meta, cnt, na, S);
+    killed = corr_point32(d, P, t.i, meta, cnt, na, S);
   }
   if (!d.sym) {
     // directed bond states: a killed point loses all its bonds (correspondence.jl:293)
@@ -579,6 +579,19 @@ static int tile_split(const DevBody& d) {
     default: { constexpr int WW = 1; CALL; } break;                \
   }
 
+// correspondence phase A: plain sums of the displacement gradient are bond-stream variant 5's
+template <bool CLS, bool COMP>
+static void launch_c_a(const DevBody& d, const LaunchCfg& c, int kstep, int grid, int smem, cudaStream_t s) {
+  const bool lin = d.kernel == KER_LINEAR;
+  if (c.fullk) {
+    if (lin) PD_TILE_LAUNCH(1, (k_c_a32s<CLS, true, true, COMP>));
+    else PD_TILE_LAUNCH(1, (k_c_a32s<CLS, true, false, COMP>));
+  } else {
+    if (lin) PD_TILE_LAUNCH(1, (k_c_a32s<CLS, false, true, COMP>));
+    else PD_TILE_LAUNCH(1, (k_c_a32s<CLS, false, false, COMP>));
+  }
+}
+
 template <bool CLS>
 static void launch_tile(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s) {
   const long long nt = (d.nslices + TILE_SLICES - 1) / TILE_SLICES;
@@ -601,12 +614,10 @@ static void launch_tile(const DevBody& d, const LaunchCfg& c, int kstep, int pha
   } else if (phase == 2) {
     if (lin) { PD_TILE_W(PD_TILE_LAUNCH(WW, (k_c_b32s<CLS, WW, true>))) }
     else { PD_TILE_W(PD_TILE_LAUNCH(WW, (k_c_b32s<CLS, WW, false>))) }
-  } else if (c.fullk) {
-    if (lin) PD_TILE_LAUNCH(1, (k_c_a32s<CLS, true, true>));
-    else PD_TILE_LAUNCH(1, (k_c_a32s<CLS, true, false>));
+  } else if (c.pipe == 5) {
+    launch_c_a<CLS, false>(d, c, kstep, grid, smem, s);
   } else {
-    if (lin) PD_TILE_LAUNCH(1, (k_c_a32s<CLS, false, true>));
-    else PD_TILE_LAUNCH(1, (k_c_a32s<CLS, false, false>));
+    launch_c_a<CLS, true>(d, c, kstep, grid, smem, s);
   }
 }
 
