@@ -56,17 +56,32 @@ DR_STRAIN = 5e-5
 # v_half_old read, v_half, v, v_half_old, b_int_old written)
 # (FP64: 128 + 176 B; FP32: b_int is 12 B, 116 + 164 B)
 B_DR_POINT = {"fp64": 304.0, "fp32": 280.0}
-# algorithmic bytes (FP32-compensated form): per directed bond the neighbour's place in its tile 2 +
-# class of its reference vector 1 + 1/8 bit (FP64 BB and OSB: place 2 + length 8 + 1/8 bit; FP64 CMat
-# nbr 4 + gathered X 24 + length 8 + 1/8 bit; energy correction, which runs without tiles: nbr 4 + xi
-# 12 + L 4 + factor 4 (FP64: 8) + 1/8 bit); per point 140 (u, v FP64 read+write, own u, b_ext/BC, parameter id, damage) + 8 for OSB
+# Bytes of the stream per directed bond in the form that a force kernel runs in, with 1/8 for the state bit.
+# On tiles the neighbour's place 2, then FP32 the class of the reference vector 1, or the vector and its
+# length 16, FP64 the length 8. Elsewhere the neighbour's number 4, then FP32 vector and length 16, FP64
+# length 8 (correspondence and the serial order also gather the neighbour's reference position, 24). The
+# energy correction's factor: 4, FP64 8.
+def bond_bytes(prec, mat, tiles, classes=0, energy=False, serial=False):
+    if prec == "fp32":
+        b = 2.0 + (1.0 if classes else 16.0) if tiles else 20.0 + (4.0 if energy else 0.0)
+    elif tiles:
+        b = 10.0
+    else:
+        b = 12.0 + (24.0 if serial or mat.startswith("C") else 0.0) + (8.0 if energy else 0.0)
+    return b + 0.125
+
+
+def bond_stream(dev, prec, mat, phase="phase_a"):
+    """(bytes per directed bond, what bounds the kernel, whether the bond classes are read) of a phase
+    of this device body as it is set up now."""
+    _, classes, on = dev.tile_info()
+    tiles = bool(on & (1 if phase == "phase_a" else 2))
+    return (bond_bytes(prec, mat, tiles, classes, dev.esc, dev.mapping()[0] == 0),
+            "issue" if tiles else "hbm", tiles and classes > 0)
+
+
+# bytes per point: 140 (u, v FP64 read+write, own u, b_ext/BC, parameter id, damage) + 8 for OSB
 # (m, theta) + 72 for CMat (F, P K^-1) + 24 with ZEMWan (the symmetric stiffness C : K^-1)
-def bond_bytes(prec, mat, energy=False):
-    if energy:
-        return {"fp32": 24.125, "fp64": 44.125}[prec]
-    return 3.125 if prec == "fp32" else 36.125 if mat.startswith("C") else 10.125
-
-
 B_POINT = {"fp32": 140.0, "fp64": 184.0}
 B_POINT_EXTRA = {"BB": 0.0, "OSB": 8.0, "C": 72.0, "CW": 96.0}
 # steps of the legs beside the timed run (per-kernel events, end to end): at most this many
@@ -653,7 +668,8 @@ def run_dr(args, rank, world, local, dist):
     # roofline: the force kernels of a step (OSB: phases A and B each stream every bond once)
     n_phase = 1 if mat == "BB" else 2
     pt = {"fp32": 64 + 8 + 16 + 4 + 4, "fp64": 128 + 8 + 32 + 4 + 4}[prec]
-    force_bytes = n_phase * (n_bonds * bond_bytes(prec, mat) + n_pts * pt)
+    streams = [bond_stream(dev, prec, mat, f"phase_{k}") for k in "ab"[:n_phase]]
+    force_bytes = sum(n_bonds * q[0] + n_pts * pt for q in streams)
     peak, peak_kind = load_peaks()
     force_ms = ms_force / args.steps
     achieved = force_bytes / (force_ms / 1e3) / 1e9
@@ -693,9 +709,9 @@ def run_dr(args, rank, world, local, dist):
                                    f"uniform tension (strain {DR_STRAIN}), dynamic relaxation step",
                        "points": n_pts, "bonds": n_bonds, "precision": prec,
                        "mapping": dict(zip(("group", "block", "pipe"), mapping)),
-                       "l2": "inputs larger than L2 (bond arrays of ~2.5 GB)",
+                       "l2": f"inputs larger than L2 (bond arrays of {n_bonds * streams[-1][0] / 1e9:.1f} GB)",
                        "parallelism": f"replicas x{world}"},
-            "roofline": {"bound": "hbm", "kernel": f"{mat.lower()} force (all phases of a step)",
+            "roofline": {"bound": streams[-1][1], "kernel": f"{mat.lower()} force (all phases of a step)",
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None, "peak_kind": peak_kind,
                          "alg_bytes_per_step": force_bytes, "ms_per_step": force_ms},
@@ -756,7 +772,8 @@ def run_halo(args, rank, world, local, dist):
     prec = args.precision
     dom = "force_b" if "force_b" in ms else "force_a"
     pt_bytes = {"fp32": 32 + 8 + 16 + 12 + 4, "fp64": 64 + 8 + 32 + 24 + 4}[prec]
-    alg = all_bonds * bond_bytes(prec, mat) + rows * pt_bytes
+    streams = [bond_stream(p.dev, prec, mat, "phase_b" if dom == "force_b" else "phase_a") for p in parts]
+    alg = sum(p.dev.info()[1] * q[0] for p, q in zip(parts, streams)) + rows * pt_bytes
     dom_ms = ms[dom] / args.steps
     peak, peak_kind = load_peaks()
     achieved = alg / (dom_ms / 1e3) / 1e9
@@ -793,7 +810,7 @@ def run_halo(args, rank, world, local, dist):
             "halo": {"ms_per_step": {k: v / args.steps for k, v in ms.items()},
                      "rows_here": rows, "halo_rows_here": halo_rows,
                      "bonds_here": all_bonds, "owned_bonds_here": owned_bonds},
-            "roofline": {"bound": "hbm", "kernel": f"{mat.lower()} {dom} (rank 0's partitions)",
+            "roofline": {"bound": streams[0][1], "kernel": f"{mat.lower()} {dom} (rank 0's partitions)",
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None, "peak_kind": peak_kind,
                          "alg_bytes_per_launch": alg, "ms_per_launch": dom_ms},
@@ -1180,7 +1197,7 @@ def main():
         pt_bytes = {"phase_a": 32 + 8 + 16 + 4 + 4, "phase_b": 32 + 8 + 16 + 12 + 4}[dom]
     else:
         pt_bytes = {"phase_a": 64 + 8 + 32 + 4 + 4, "phase_b": 64 + 8 + 32 + 24 + 4}[dom]
-    b_bond = bond_bytes(prec, mat, args.correction == "energy")
+    b_bond, bound, by_class = bond_stream(dev, prec, mat, dom)
     alg_bytes = n_bonds * b_bond + n_pts * pt_bytes
     achieved = alg_bytes / (dom_ms / 1e3) / 1e9
     # DRAM traffic per launch from the committed ncu capture, scaled by the bond count
@@ -1189,7 +1206,7 @@ def main():
         with open(os.path.join(ROOT, "profiles", "traffic.json")) as f:
             tb = json.load(f)["dram_bytes_per_bond"]
         key = {"phase_a": f"{mat.lower()}_phase_a", "phase_b": f"{mat.lower()}_phase_b"}[dom]
-        if prec == "fp32" and key in tb:
+        if prec == "fp32" and by_class and key in tb:  # the capture's form
             traffic = tb[key] * n_bonds
     except Exception:
         traffic = None
@@ -1265,7 +1282,7 @@ def main():
                        "parallelism": f"replicas x{world}"},
             # on tiles issue slots and shared memory bound the force kernels; the bytes are those of
             # the stream that they read
-            "roofline": {"bound": "hbm" if args.correction == "energy" else "issue",
+            "roofline": {"bound": bound,
                          "kernel": f"{mat.lower()} force {dom}",
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,

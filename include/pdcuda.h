@@ -294,6 +294,11 @@ pd_status pd_set_pipeline(pd_handle *h, int32_t pipe);
 /* The current mapping (group 0 = serial order), block size and bond-stream variant. */
 pd_status pd_get_mapping(pd_handle *h, int32_t *group, int32_t *block, int32_t *pipe);
 
+/* Which form the force kernels run in: the points of the largest tile (0: the body has no tiles), the number
+ * of bond classes (0: none, FP64 or not a regular lattice) and the phases that run on tiles, 1 for the first
+ * force kernel (BB: the only one) plus 2 for the second. Any output may be NULL. */
+pd_status pd_tile_info(pd_handle *h, int32_t *tile_points, int32_t *classes, int32_t *phases);
+
 /* Enables CUDA-graph capture of blocks of `steps_per_graph` steps (0 disables). */
 pd_status pd_set_graph(pd_handle *h, int32_t steps_per_graph);
 

@@ -1074,6 +1074,11 @@ extern "C" pd_status pd_set_param_timesteps(pd_handle* h, const double* dtp) {
   return PD_OK;
 }
 
+// bond-stream variants 1 to 3 where they apply
+static bool runs_tma(const pd_handle* h) {
+  return h->cfg.pipe >= 1 && h->cfg.pipe <= 3 && !h->d.sc32 && tma_supported(h->d);
+}
+
 static int launch_force(pd_handle* h, int kstep, int phase) {
   int k;
   // FP32 OSB / CMat: the first phase-A launch after bond states changed outside the kernels sums
@@ -1083,7 +1088,7 @@ static int launch_force(pd_handle* h, int kstep, int phase) {
   h->cfg.fullk = fullk ? 1 : 0;
   if (fullk) { h->kfull = false; h->version++; }
   if (h->precision == PD_PREC_FP64) k = launch_force64(h->d, h->cfg, kstep, phase, h->stream);
-  else if (h->cfg.pipe >= 1 && h->cfg.pipe <= 3 && !h->d.sc32 && tma_supported(h->d))
+  else if (runs_tma(h))
     k = launch_force32_tma(h->d, h->cfg.pipe, kstep, phase, h->stream);
   else k = launch_force32(h->d, h->cfg, kstep, phase, h->stream);
   h->launches += k;
@@ -1646,6 +1651,20 @@ extern "C" pd_status pd_get_mapping(pd_handle* h, int32_t* group, int32_t* block
   if (group) *group = h->cfg.exact ? 0 : h->cfg.group;
   if (block) *block = h->cfg.block;
   if (pipe) *pipe = h->cfg.pipe;
+  return PD_OK;
+}
+
+extern "C" pd_status pd_tile_info(pd_handle* h, int32_t* tile_points, int32_t* classes, int32_t* phases) {
+  if (!h) return fail(PD_ERR_ARG, "handle is NULL");
+  int on = 0;
+  for (int phase = 1; phase <= (h->material == PD_MAT_BB ? 1 : 2); phase++) {
+    const bool t = h->precision == PD_PREC_FP64 ? !h->cfg.exact && tile64_supported(h->d, phase)
+                                                : !runs_tma(h) && force32_on_tiles(h->d, phase);
+    if (t) on |= phase;
+  }
+  if (tile_points) *tile_points = h->d.tile_pt ? h->d.tile_cap : 0;
+  if (classes) *classes = h->d.ncls;
+  if (phases) *phases = on;
   return PD_OK;
 }
 

@@ -1053,7 +1053,7 @@ static int launch_osb32(const DevBody& d, const LaunchCfg& c, int G, int grid, i
 // The tile kernels (pd_tile32.cu) run wherever the packed kernels' conditions hold and the body has
 // tiles, whatever the bond-stream variant: they were the fastest of all variants at every size
 // measured (pd_tile32.cu).
-static bool on_tiles(const DevBody& d, int phase) {
+bool force32_on_tiles(const DevBody& d, int phase) {
   return packed_supported(d, phase) && tile32_supported(d, phase);
 }
 
@@ -1065,7 +1065,7 @@ int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, c
   if (d.material == MAT_BB && !A) return 0;
   if (phase == 0 && d.material != MAT_BB)
     return launch_force32(d, c, kstep, 1, s) + launch_force32(d, c, kstep, 2, s);
-  if (on_tiles(d, A ? 1 : 2)) {
+  if (force32_on_tiles(d, A ? 1 : 2)) {
     launch_tile32(d, c, kstep, A ? 1 : 2, s);
     return 1;
   }

@@ -125,6 +125,8 @@ cudaError_t build_classes(const DevBody& d, long long nslots, unsigned** cls, fl
                           cudaStream_t s);
 // the tile kernels (pd_tile32.cu) of a phase (1: the first, 2: the second) of an FP32 body
 bool tile32_supported(const DevBody& d, int phase);
+// whether launch_force32 takes them (pd_force32.cu)
+bool force32_on_tiles(const DevBody& d, int phase);
 void launch_tile32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s);
 
 // sliced bond layout and bond-array helpers (pd_layout.cu)

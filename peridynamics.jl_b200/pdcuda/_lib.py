@@ -51,7 +51,7 @@ EXPORTS = (
     "pd_mpnn_infer", "pd_mpnn_loss_grad", "pd_mpnn_spectral_grad", "pd_mpnn_zero_grad",
     "pd_mpnn_adam",
     "pd_osb_force_static", "pd_static_last_error",
-    "pd_group_create", "pd_group_run_vv", "pd_group_destroy",
+    "pd_group_create", "pd_group_run_vv", "pd_group_destroy", "pd_tile_info",
 )
 
 
@@ -190,6 +190,7 @@ def lib():
         "pd_group_create": [vp, i32, vp],
         "pd_group_run_vv": [vp, i64, i64, dbl, i32, vp],
         "pd_group_destroy": [vp],
+        "pd_tile_info": [vp, vp, vp, vp],
     }
     for name, args in sig.items():
         f = getattr(L, name)

@@ -310,6 +310,13 @@ class DeviceBody:
         L.check(L.lib().pd_get_mapping(self.h, C.byref(g), C.byref(b), C.byref(p)), "pd_get_mapping")
         return g.value, b.value, p.value
 
+    def tile_info(self):
+        """(points of the largest tile, bond classes, phases that run on tiles: 1 for the first
+        force kernel plus 2 for the second); 0 where the body has none."""
+        t, c, p = C.c_int32(), C.c_int32(), C.c_int32()
+        L.check(L.lib().pd_tile_info(self.h, C.byref(t), C.byref(c), C.byref(p)), "pd_tile_info")
+        return t.value, c.value, p.value
+
     def autotune(self):
         g, b = C.c_int32(), C.c_int32()
         L.check(L.lib().pd_autotune(self.h, C.byref(g), C.byref(b)), "pd_autotune")
