@@ -286,9 +286,11 @@ pd_status pd_set_mapping(pd_handle *h, int32_t group, int32_t block);
  * lane per point and one parameter set; phase B needs symmetric bond states and, for CMat,
  * ZEMSilling; BB and OSB need no surface correction; where they do not apply the phase runs
  * as 4, CMat as 0; same FP32 form, roundings differ in the order of a few operations).
- * pd_autotune times all that apply. Bodies with one lane per point to which 5 applies run 0, 4 and 5
- * on tiles of points in shared memory instead (the same results for all three), unless a tile would
- * need more than 4095 points. */
+ * pd_autotune times all that apply. With one lane per point and where 5 applies, 0, 4 and 5 run the
+ * packed arithmetic on tiles of points in shared memory, or from global memory where a tile would need more
+ * than 4095 points or more shared memory than a block has (correspondence phase B: about 3100 points), or
+ * where there is no memory for the tiles: the same results either way and for 0, 4 and 5, but that CMat sums
+ * the displacement gradient with compensation unless 5 asks for plain sums. */
 pd_status pd_set_pipeline(pd_handle *h, int32_t pipe);
 
 /* The current mapping (group 0 = serial order), block size and bond-stream variant. */

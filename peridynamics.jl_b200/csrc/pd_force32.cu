@@ -18,9 +18,9 @@
 // FP32 for millimetre lattices). The stress formulas are the reference's, rewritten in
 // terms of E = (H + H^T + H^T H) / 2 without cancelling subtractions.
 //
-// Bodies with tiles (one lane per point, bond-stream variants 0, 4 and 5) run pd_tile32.cu; the kernels
-// here serve the other lane groups, ZEMWan's phase B, directed bond states, several parameter sets in
-// phase B and EnergySurfaceCorrection.
+// One lane per point and one parameter set runs pd_tile32.cu, or where its tiles do not fit pd_force32_pk.cu and
+// the packed correspondence kernels below; the other kernels here serve lane groups, ZEMWan's phase B,
+// directed bond states, several parameter sets and EnergySurfaceCorrection.
 #include "pd_bond32.cuh"
 #include "pd_common.cuh"
 #include "pd_launch.h"
@@ -786,11 +786,11 @@ __global__ void __launch_bounds__(256, PD_MINB_CB) k_c_b32(DevBody d, int kstep)
 }
 
 // -------------------------------------------------------------------------------------------
-// CMat phases with packed pairs and the next row pair's bond stream in flight (bond-stream
-// variant 5; one lane per point, one parameter set; phase B for symmetric bond states). The
+// CMat phases with packed pairs and the next row pair's bond stream in flight (one lane per point, one
+// parameter set, bodies whose tiles do not fit; phase B for symmetric bond states). The
 // per-bond sums are those of k_c_a32 / k_c_b32: the x and y rows of every 3x3 sum are one
-// packed pair, z is scalar (the shape-tensor and force sums compensated, the
-// displacement-gradient sums of phase A plain); bond states select the contributions (inactive bonds
+// packed pair, z is scalar (the shape-tensor and force sums compensated, the displacement-gradient sums of
+// phase A too unless bond-stream variant 5 asks for plain ones); bond states select the contributions (inactive bonds
 // and padding slots gather their own point and add zero). The per-point epilogue of phase A is
 // k_c_a32's. Phase B: with one influence value for both directions, t_ij + the term of j is
 // w V_j ((A_i + A_j) xi + (beta_i + beta_j) du).
@@ -806,8 +806,8 @@ __global__ void __launch_bounds__(256, PD_MINB_CB) k_c_b32(DevBody d, int kstep)
 #define PD_MINB_CQB 3
 #endif
 
-template <bool FULLK, bool LIN>
-__global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kstep) {
+template <bool FULLK, bool LIN, bool COMP>
+__global__ void __launch_bounds__(256, COMP ? 2 : PD_MINB_CQA) k_c_a32q(DevBody d, int kstep) {
   using namespace pack;
   if (d.ctrl->err) return;
   const int lane = threadIdx.x & 31;
@@ -829,7 +829,7 @@ __global__ void __launch_bounds__(256, PD_MINB_CQA) k_c_a32q(DevBody d, int kste
     const int* pn = d.nbr + sbase + lane;
     const float4* pg = d.geo + sbase + lane;
     unsigned* pw = d.bits + (sbase >> 5);
-    CorrSums<FULLK, false> S;
+    CorrSums<FULLK, COMP> S;
     int na = 0;
     int nj0 = self, nj1 = self;
     float4 ng0 = make_float4(0.f, 0.f, 0.f, 1.f), ng1 = ng0;
@@ -1050,18 +1050,30 @@ static int launch_osb32(const DevBody& d, const LaunchCfg& c, int G, int grid, i
   return launches;
 }
 
-// The tile kernels (pd_tile32.cu) run wherever the packed kernels' conditions hold and the body has
-// tiles, whatever the bond-stream variant: they were the fastest of all variants at every size
-// measured (pd_tile32.cu).
+// One lane per point and one parameter set: the packed arithmetic whatever the bond-stream variant
+// (1 to 3 apart), on tiles (pd_tile32.cu) where they fit and from global memory else. On tiles it was the
+// fastest of all variants at every size measured; and a body and its partitions, which may lie on
+// different sides of that limit, have the same results.
 bool force32_on_tiles(const DevBody& d, int phase) {
   return packed_supported(d, phase) && tile32_supported(d, phase);
+}
+
+template <bool COMP>
+static void launch_c_a32q(const DevBody& d, const LaunchCfg& c, int grid, int kstep, cudaStream_t s) {
+  const bool lin = d.kernel == KER_LINEAR;
+  if (c.fullk) {
+    if (lin) k_c_a32q<true, true, COMP><<<grid, c.block, 0, s>>>(d, kstep);
+    else k_c_a32q<true, false, COMP><<<grid, c.block, 0, s>>>(d, kstep);
+  } else {
+    if (lin) k_c_a32q<false, true, COMP><<<grid, c.block, 0, s>>>(d, kstep);
+    else k_c_a32q<false, false, COMP><<<grid, c.block, 0, s>>>(d, kstep);
+  }
 }
 
 int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, cudaStream_t s) {
   const int G = d.lg;
   const int grid = grid_for32(d.nslices, c.block);
   const bool A = phase != 2, B = phase != 1;
-  int launches = 0;
   if (d.material == MAT_BB && !A) return 0;
   if (phase == 0 && d.material != MAT_BB)
     return launch_force32(d, c, kstep, 1, s) + launch_force32(d, c, kstep, 2, s);
@@ -1069,43 +1081,30 @@ int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, c
     launch_tile32(d, c, kstep, A ? 1 : 2, s);
     return 1;
   }
+  if (pk_supported(d, A ? 1 : 2)) return launch_force32_pk(d, c, kstep, A ? 1 : 2, s);
+  LaunchCfg c4 = c;
+  if (c.pipe == 5) c4.pipe = 4;  // the two-row kernels where the packed ones do not apply
   if (d.material == MAT_BB) {
-    if (c.pipe == 5 && pk_supported(d, 1)) return launch_force32_pk(d, c, kstep, 1, s);
-    LaunchCfg c4 = c;
-    if (c.pipe == 5) c4.pipe = 4;   // the two-row kernel where the packed one does not apply
     if (d.sc32) launch_bb32<true>(d, c4, G, grid, kstep, s);
     else launch_bb32<false>(d, c4, G, grid, kstep, s);
     return 1;
   }
   if (d.material == MAT_OSB) {
-    if (c.pipe == 5) {
-      // the packed kernels where they apply, the two-row kernels for the other phase
-      LaunchCfg c4 = c;
-      c4.pipe = 4;
-      const bool pa = A && pk_supported(d, 1), pb = B && pk_supported(d, 2);
-      if (A) launches += pa ? launch_force32_pk(d, c, kstep, 1, s)
-                            : (d.sc32 ? launch_osb32<true>(d, c4, G, grid, kstep, true, false, s)
-                                      : launch_osb32<false>(d, c4, G, grid, kstep, true, false, s));
-      if (B) launches += pb ? launch_force32_pk(d, c, kstep, 2, s)
-                            : (d.sc32 ? launch_osb32<true>(d, c4, G, grid, kstep, false, true, s)
-                                      : launch_osb32<false>(d, c4, G, grid, kstep, false, true, s));
-      return launches;
-    }
-    if (d.sc32) return launch_osb32<true>(d, c, G, grid, kstep, A, B, s);
-    return launch_osb32<false>(d, c, G, grid, kstep, A, B, s);
+    if (d.sc32) return launch_osb32<true>(d, c4, G, grid, kstep, A, B, s);
+    return launch_osb32<false>(d, c4, G, grid, kstep, A, B, s);
   }
   const bool lin = d.kernel == KER_LINEAR;
-  if (A && c.pipe == 5 && cq_supported(d, 1)) {
-    if (c.fullk) {
-      if (lin) k_c_a32q<true, true><<<grid, c.block, 0, s>>>(d, kstep);
-      else k_c_a32q<true, false><<<grid, c.block, 0, s>>>(d, kstep);
+  if (cq_supported(d, A ? 1 : 2)) {
+    if (B) {
+      if (lin) k_c_b32q<true><<<grid, c.block, 0, s>>>(d, kstep);
+      else k_c_b32q<false><<<grid, c.block, 0, s>>>(d, kstep);
+    } else if (c.pipe == 5) {
+      launch_c_a32q<false>(d, c, grid, kstep, s);
     } else {
-      if (lin) k_c_a32q<false, true><<<grid, c.block, 0, s>>>(d, kstep);
-      else k_c_a32q<false, false><<<grid, c.block, 0, s>>>(d, kstep);
+      launch_c_a32q<true>(d, c, grid, kstep, s);
     }
-    launches++;
   } else if (A) {
-    if (d.kernel == KER_LINEAR) {
+    if (lin) {
       if (c.fullk) { PD_DISPATCH_G(G, (k_c_a32<GG, true, true><<<grid, c.block, 0, s>>>(d, kstep))); }
       else { PD_DISPATCH_G(G, (k_c_a32<GG, false, true><<<grid, c.block, 0, s>>>(d, kstep))); }
     } else if (c.fullk) {
@@ -1113,25 +1112,15 @@ int launch_force32(const DevBody& d, const LaunchCfg& c, int kstep, int phase, c
     } else {
       PD_DISPATCH_G(G, (k_c_a32<GG, false, false><<<grid, c.block, 0, s>>>(d, kstep)));
     }
-    launches++;
+  } else if (d.zem == ZEM_WAN) {
+    if (d.sym) { PD_DISPATCH_G(G, (k_c_b32<GG, true, true><<<grid, c.block, 0, s>>>(d, kstep))); }
+    else { PD_DISPATCH_G(G, (k_c_b32<GG, false, true><<<grid, c.block, 0, s>>>(d, kstep))); }
+  } else if (d.sym) {
+    PD_DISPATCH_G(G, (k_c_b32<GG, true, false><<<grid, c.block, 0, s>>>(d, kstep)));
+  } else {
+    PD_DISPATCH_G(G, (k_c_b32<GG, false, false><<<grid, c.block, 0, s>>>(d, kstep)));
   }
-  const bool wan = d.zem == ZEM_WAN;
-  if (B && c.pipe == 5 && cq_supported(d, 2)) {
-    if (lin) k_c_b32q<true><<<grid, c.block, 0, s>>>(d, kstep);
-    else k_c_b32q<false><<<grid, c.block, 0, s>>>(d, kstep);
-    launches++;
-  } else if (B) {
-    if (wan) {
-      if (d.sym) { PD_DISPATCH_G(G, (k_c_b32<GG, true, true><<<grid, c.block, 0, s>>>(d, kstep))); }
-      else { PD_DISPATCH_G(G, (k_c_b32<GG, false, true><<<grid, c.block, 0, s>>>(d, kstep))); }
-    } else if (d.sym) {
-      PD_DISPATCH_G(G, (k_c_b32<GG, true, false><<<grid, c.block, 0, s>>>(d, kstep)));
-    } else {
-      PD_DISPATCH_G(G, (k_c_b32<GG, false, false><<<grid, c.block, 0, s>>>(d, kstep)));
-    }
-    launches++;
-  }
-  return launches;
+  return 1;
 }
 
 }  // namespace pd

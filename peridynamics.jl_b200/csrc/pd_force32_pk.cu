@@ -1,6 +1,6 @@
-// pd_force32_pk.cu -- FP32-compensated OSB force kernels with fewer instructions per bond and
-// the bond stream of the next row pair in flight (bond-stream variant 5: one lane per point,
-// the sliced layout of G = 1).
+// pd_force32_pk.cu -- FP32-compensated BB and OSB force kernels with fewer instructions per bond and
+// the bond stream of the next row pair in flight (one lane per point, the sliced layout of G = 1, bodies
+// whose tiles do not fit).
 //
 // The two-row kernels (pd_force32.cu) issue about 93 (phase A) and 116 (phase B) warp
 // instructions per bond row. These compute the same quantities with 75 / 68:
