@@ -1472,6 +1472,25 @@ extern "C" pd_status pd_set_mapping(pd_handle* h, int32_t group, int32_t block) 
   return PD_OK;
 }
 
+// the phases that run on tiles: 1 for the first force kernel plus 2 for the second
+static int tile_phases(const pd_handle* h) {
+  int on = 0;
+  for (int phase = 1; phase <= (h->material == PD_MAT_BB ? 1 : 2); phase++) {
+    const bool t = h->precision == PD_PREC_FP64 ? !h->cfg.exact && tile64_supported(h->d, phase)
+                                                : !runs_tma(h) && force32_on_tiles(h->d, phase);
+    if (t) on |= phase;
+  }
+  return on;
+}
+
+extern "C" pd_status pd_tile_info(pd_handle* h, int32_t* tile_points, int32_t* classes, int32_t* phases) {
+  if (!h) return fail(PD_ERR_ARG, "handle is NULL");
+  if (tile_points) *tile_points = h->d.tile_pt ? h->d.tile_cap : 0;
+  if (classes) *classes = h->d.ncls;
+  if (phases) *phases = tile_phases(h);
+  return PD_OK;
+}
+
 extern "C" pd_status pd_autotune(pd_handle* h, int32_t* group_out, int32_t* block_out) {
   if (!h) return fail(PD_ERR_ARG, "handle is NULL");
   PD_CUDA(cudaSetDevice(h->device));
@@ -1492,31 +1511,46 @@ extern "C" pd_status pd_autotune(pd_handle* h, int32_t* group_out, int32_t* bloc
     cudaEventElapsedTime(out, e0, e1);
     return PD_OK;
   };
-  const int groups[] = {1, 4, 32};
-  const int blocks[] = {128, 256};
+  auto give_up = [&](pd_status st) {
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    return st;
+  };
   // force evaluations are idempotent at fixed positions: bonds that broke stay broken and
   // every output is recomputed
-  for (int G : groups) {
-    pd_status st = relayout(h, G);
-    if (st == PD_ERR_OOM) { cudaGetLastError(); continue; }  // no room for a second layout
-    if (st != PD_OK) { cudaEventDestroy(e0); cudaEventDestroy(e1); return st; }
-    const bool tma = h->precision == PD_PREC_FP32_KAHAN && G == 1 && tma_supported(h->d);
-    const bool two = h->precision == PD_PREC_FP32_KAHAN && h->material != PD_MAT_CMAT;
-    const bool packed = h->precision == PD_PREC_FP32_KAHAN && G == 1 && packed_supported(h->d, 1);
-    // candidates: blocks of 128 / 256 with plain loads, then (FP32 BB / OSB) the two-row
-    // kernels, then (one lane per point) the TMA-staged bond stream, then (FP32 OSB, one lane
-    // per point) the packed-pair kernels
-    for (int v = 0; v < 9; v++) {
-      if ((v == 2 || v == 3) && !two) continue;
-      if (v >= 4 && v < 7 && !tma) continue;
-      if (v >= 7 && !packed) continue;
-      const int B = v < 4 ? blocks[v % 2] : v < 7 ? 128 : blocks[v - 7];
-      h->cfg.group = G; h->cfg.block = B; h->cfg.exact = false;
-      h->cfg.pipe = v < 2 ? 0 : v < 4 ? 4 : v < 7 ? v - 3 : 5;
-      float ms;
-      pd_status ts = time_cfg(&ms);
-      if (ts != PD_OK) { cudaEventDestroy(e0); cudaEventDestroy(e1); return ts; }
-      cands.push_back({ms, h->cfg});
+  const bool f32 = h->precision == PD_PREC_FP32_KAHAN, corr = h->material == PD_MAT_CMAT;
+  for (int G : {1, 4, 32}) {
+    // the variants to time: plain loads, then (FP32 BB / OSB) the two-row kernels, then (one lane per point)
+    // the TMA-staged bond stream and the packed kernels
+    std::vector<int> pipes{0};
+    if (f32 && !corr) pipes.push_back(4);
+    if (f32 && G == 1) {
+      if (!corr) pipes.insert(pipes.end(), {1, 2, 3});
+      pipes.push_back(5);
+    }
+    for (int pipe : pipes) {
+      h->cfg.group = G; h->cfg.exact = false; h->cfg.pipe = pipe;
+      pd_status st = relayout(h, G);
+      if (st == PD_ERR_OOM) { cudaGetLastError(); break; }  // no room for a second layout
+      if (st != PD_OK) return give_up(st);
+      const bool tma = pipe >= 1 && pipe <= 3;
+      if (tma && !tma_supported(h->d)) continue;
+      if (pipe == 5 && !packed_supported(h->d, 1)) continue;
+      // where every phase runs the packed kernels the plain variants are the same ones (correspondence: 0
+      // has sums of its own); on tiles the block size is the tile's
+      const bool bb = h->material == PD_MAT_BB;
+      if (G == 1 && f32 && !corr && (pipe == 0 || pipe == 4) && packed_supported(h->d, 1) &&
+          (bb || packed_supported(h->d, 2)))
+        continue;
+      const bool tiles = tile_phases(h) == (bb ? 1 : 3);
+      for (int B : {128, 256}) {
+        if (B == 256 && (tma || tiles)) continue;
+        h->cfg.block = B;
+        float ms;
+        st = time_cfg(&ms);
+        if (st != PD_OK) return give_up(st);
+        cands.push_back({ms, h->cfg});
+      }
     }
   }
   // the three fastest are timed twice more, interleaved, and keep their best time: one window
@@ -1525,11 +1559,11 @@ extern "C" pd_status pd_autotune(pd_handle* h, int32_t* group_out, int32_t* bloc
   if (cands.size() > 3) cands.resize(3);
   for (int round = 0; round < 2 && cands.size() > 1; round++)
     for (auto& c : cands) {
-      if (relayout(h, c.c.group) != PD_OK) { cudaGetLastError(); continue; }
       h->cfg = c.c;
+      if (relayout(h, c.c.group) != PD_OK) { cudaGetLastError(); continue; }
       float ms;
       pd_status ts = time_cfg(&ms);
-      if (ts != PD_OK) { cudaEventDestroy(e0); cudaEventDestroy(e1); return ts; }
+      if (ts != PD_OK) return give_up(ts);
       c.ms = std::min(c.ms, ms);
     }
   cudaEventDestroy(e0);
@@ -1538,8 +1572,8 @@ extern "C" pd_status pd_autotune(pd_handle* h, int32_t* group_out, int32_t* bloc
   float best = INFINITY;
   for (const auto& c : cands)
     if (c.ms < best) { best = c.ms; bestc = c.c; }
-  PD_TRY(relayout(h, bestc.group));
   h->cfg = bestc;
+  PD_TRY(relayout(h, bestc.group));
   drop_graphs(h);
   if (group_out) *group_out = bestc.group;
   if (block_out) *block_out = bestc.block;
@@ -1651,20 +1685,6 @@ extern "C" pd_status pd_get_mapping(pd_handle* h, int32_t* group, int32_t* block
   if (group) *group = h->cfg.exact ? 0 : h->cfg.group;
   if (block) *block = h->cfg.block;
   if (pipe) *pipe = h->cfg.pipe;
-  return PD_OK;
-}
-
-extern "C" pd_status pd_tile_info(pd_handle* h, int32_t* tile_points, int32_t* classes, int32_t* phases) {
-  if (!h) return fail(PD_ERR_ARG, "handle is NULL");
-  int on = 0;
-  for (int phase = 1; phase <= (h->material == PD_MAT_BB ? 1 : 2); phase++) {
-    const bool t = h->precision == PD_PREC_FP64 ? !h->cfg.exact && tile64_supported(h->d, phase)
-                                                : !runs_tma(h) && force32_on_tiles(h->d, phase);
-    if (t) on |= phase;
-  }
-  if (tile_points) *tile_points = h->d.tile_pt ? h->d.tile_cap : 0;
-  if (classes) *classes = h->d.ncls;
-  if (phases) *phases = on;
   return PD_OK;
 }
 

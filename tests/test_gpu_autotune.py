@@ -1,0 +1,32 @@
+"""What pd_autotune times: every kernel once, not under each of its names."""
+import numpy as np
+import pytest
+
+import pdcuda as pd
+from helpers import deform, oracle_body
+from test_gpu_tiles import MATERIALS, box
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("name", list(MATERIALS))
+def test_autotune_times_a_kernel_once(name):
+    """One lane per point: the packed kernels on tiles (correspondence: both kinds of sums) and three staged
+    variants (BB, OSB); 4 and 32 lanes: one- and (BB, OSB) two-row kernels with two block sizes. Six
+    evaluations each, and two more rounds of the fastest three."""
+    body = box(MATERIALS[name](), 17, 9, 6, 3.015)
+    dev = pd.DeviceBody(body, precision="fp32")
+    u = deform(body._pos)
+    dev.set_state(displacement=u)
+    before = dev.launch_count()
+    dev.autotune()
+    corr = name == "C"
+    candidates = 2 + 2 * 2 if corr else 1 + 3 + 2 * 4
+    per = 1 if name == "BB" else 2
+    assert dev.launch_count() - before == 6 * per * (candidates + 2 * 3)
+    ob = oracle_body(body)
+    ob.pos[:] = body._pos + u
+    ob.force_density()
+    dev.force()
+    assert np.abs(dev.field("b_int").T - ob.b_int).max() < 2e-5 * np.abs(ob.b_int).max()
+    dev.close()
