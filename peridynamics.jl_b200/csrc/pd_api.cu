@@ -149,6 +149,17 @@ static pd_status check_symmetry(pd_handle* h) {
   return PD_OK;
 }
 
+// Whether the points of the one-lane layout take places that suit tiles (pd_tiles.cu). The kernels that
+// know no tiles are slower in that order (us a step, places / the points' own order, OSB 192,000 points: two
+// parameter sets 651 / 547, the staged stream of variant 2 510 / 457, surface correction 426 / 359). ZEMWan
+// and directed bond states have their first phase on tiles and are not (variant 0, 192,000 points, against
+// the one-row kernels on the points' own order: 417 / 466 and 446 / 466).
+static bool wants_places(const pd_handle* h) {
+  if (h->multi || h->d.sc32 || h->d.sc64 || h->esc) return false;
+  if (h->cfg.pipe >= 1 && h->cfg.pipe <= 3) return false;
+  return h->precision != PD_PREC_FP64 || h->material != PD_MAT_CMAT;
+}
+
 // Bodies with one lane per point gather from tiles in shared memory (FP64: BB and OSB) and, in FP32
 // on a regular lattice, read a bond's geometry as one byte. Both are made once per layout; a body without tiles or
 // classes, or without the memory for them, runs the kernels that its bond-stream variant names.
@@ -202,7 +213,7 @@ static pd_status finish_create(pd_handle* h, int* dnbr_csr, const double* dL, co
   }
   long long* soff = nullptr;
   long long ns = 0, nslots = 0;
-  if (h->precision != PD_PREC_FP64 || h->material != PD_MAT_CMAT) {
+  if (wants_places(h)) {
     PD_CUDA(build_places(h->d, h->grid, &h->pt, &h->place, h->stream));
     h->allocs.push_back(h->pt);
     h->allocs.push_back(h->place);
@@ -316,15 +327,17 @@ static pd_status finish_create(pd_handle* h, int* dnbr_csr, const double* dL, co
   return PD_OK;
 }
 
-// moves every bond array into the layout with G lanes per point
+// moves every bond array into the layout with G lanes per point, one lane in the order that the handle's
+// kernels want
 static pd_status relayout(pd_handle* h, int G) {
-  if (G == h->d.lg) return PD_OK;
+  const bool places = G == 1 && wants_places(h) && h->pt != nullptr;
+  if (G == h->d.lg && places == (h->d.pt != nullptr)) return PD_OK;
   PD_CUDA(cudaStreamSynchronize(h->stream));
   DevBody a = h->d, b = h->d;
   long long* soff = nullptr;
   long long ns = 0, nslots = 0;
-  b.pt = G == 1 ? h->pt : nullptr;
-  b.place = G == 1 ? h->place : nullptr;
+  b.pt = places ? h->pt : nullptr;
+  b.place = places ? h->place : nullptr;
   PD_CUDA(build_slices(h->n, h->d.off, b.pt, G, &soff, &ns, &nslots, h->stream));
   h->allocs.push_back(soff);
   b.soff = soff;
@@ -1454,10 +1467,10 @@ extern "C" pd_status pd_set_mapping(pd_handle* h, int32_t group, int32_t block) 
   if (group == 0) {
     if (h->precision != PD_PREC_FP64) return fail(PD_ERR_ARG, "the serial-order mapping (group 0) is FP64 only");
     PD_CUDA(cudaSetDevice(h->device));
+    h->cfg.pipe = 0;
     PD_TRY(relayout(h, 1));
     h->cfg.exact = true;
     h->cfg.group = 1;
-    h->cfg.pipe = 0;
   } else {
     if (group != 1 && group != 2 && group != 4 && group != 8 && group != 16 && group != 32)
       return fail(PD_ERR_ARG, "group must be 0, 1, 2, 4, 8, 16 or 32");
@@ -1699,7 +1712,17 @@ extern "C" pd_status pd_set_pipeline(pd_handle* h, int32_t pipe) {
     return fail(PD_ERR_ARG, "the staged bond stream needs the FP32 path, one lane per point and BB or OSB");
   h->cfg.pipe = pipe;
   drop_graphs(h);
-  return PD_OK;
+  const pd_status st = relayout(h, h->d.lg);
+  if (st == PD_ERR_OOM) { cudaGetLastError(); return PD_OK; }  // any order will do
+  return st;
+}
+
+// pd_esc_init: the bond factors have no place in the tiles
+pd_status pd_without_tiles(pd_handle* h) {
+  h->esc = true;
+  const pd_status st = relayout(h, h->d.lg);
+  if (st == PD_ERR_OOM) { cudaGetLastError(); return PD_OK; }
+  return st;
 }
 
 // helpers shared with pd_nk.cu

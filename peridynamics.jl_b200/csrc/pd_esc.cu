@@ -183,6 +183,7 @@ extern "C" pd_status pd_esc_init(pd_handle* h, int32_t what) {
     return pd_fail(PD_ERR_UNSUPPORTED, "EnergySurfaceCorrection needs BBMaterial or OSBMaterial");
   PD_CUDA(cudaSetDevice(h->device));
   if (h->n == 0) return PD_OK;
+  PD_TRY(pd_without_tiles(h));
   if (!h->d.mf) {
     double* mf = nullptr;
     PD_TRY(dalloc(h, &mf, 3 * h->n));

@@ -70,6 +70,7 @@ struct pd_handle {
   // FP32 OSB / CMat: the stored weighted volumes / shape tensors are stale (bond states
   // changed outside the kernels)
   bool kfull = true;
+  bool esc = false;          // pd_esc_init was called
   bool tiles_tried = false;  // tiles and bond classes were looked for in the current layout
   pd::PlaceGrid grid{};      // of the places of the one-lane layout
   int* pt = nullptr;         // those places (kept while a lane-group layout is in use)
@@ -128,5 +129,6 @@ inline void dfree(pd_handle* h, void* p) {
 // helpers implemented in pd_api.cu
 pd_status pd_set_ctrl(pd_handle* h, size_t off, const void* src, size_t bytes);
 pd_status pd_clear_error(pd_handle* h);
+pd_status pd_without_tiles(pd_handle* h);
 pd_status pd_check_err(pd_handle* h);
 int pd_launch_force(pd_handle* h, int kstep, int phase);
