@@ -304,6 +304,12 @@ pd_status pd_tile_info(pd_handle *h, int32_t *tile_points, int32_t *classes, int
 /* Enables CUDA-graph capture of blocks of `steps_per_graph` steps (0 disables). */
 pd_status pd_set_graph(pd_handle *h, int32_t steps_per_graph);
 
+/* The elementary FP64 functions of the force kernels off the serial order on n host values, and CUDA's own
+ * beside them: 1 / sqrt(x), 1 / x, sqrt(x), the length sqrt(x) of a bond of reference length y, x / y. */
+enum { PD_EVAL_RSQRT = 0, PD_EVAL_RCP = 1, PD_EVAL_SQRT = 2, PD_EVAL_LENGTH = 3, PD_EVAL_QUOTIENT = 4,
+       PD_EVAL_CUDA_RSQRT = 5, PD_EVAL_CUDA_SQRT = 6, PD_EVAL_CUDA_QUOTIENT = 7 };
+pd_status pd_eval64(int32_t op, int64_t n, const double *x, const double *y, double *out, int32_t device);
+
 /* Sizes: points, bonds, and 1 if the fast symmetric-pair bond mode is active. */
 pd_status pd_info(pd_handle *h, int64_t *n_points, int64_t *n_bonds, int32_t *symmetric);
 

@@ -35,7 +35,8 @@ __device__ __forceinline__ bool class_same(const uint4& a, const uint4& b) {
   return a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w;
 }
 
-// a nonzero 64-bit fingerprint (multiply and xor-shift over the words)
+// a nonzero 64-bit fingerprint: the words through the mixing steps of splitmix64 (Steele, Lea and Flood, Fast
+// splittable pseudorandom number generators, 2014)
 __device__ __forceinline__ unsigned long long class_print(const uint4& r) {
   const unsigned v[4] = {r.x, r.y, r.z, r.w};
   unsigned long long h = 0x9E3779B97F4A7C15ull;

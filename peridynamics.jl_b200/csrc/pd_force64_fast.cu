@@ -8,9 +8,8 @@
 // point fills only a part.
 //
 //   - One reciprocal square root per bond. g = 1 / sqrt(l^2 L^2) gives 1 / (l L) directly and
-//     l = l^2 L g after one correction (the residual l^2 - l*l, exact in an fma, times 1 / 2 l):
-//     the square root rounded to nearest but for arguments within 2^-105 of a midpoint. l^2 is
-//     formed as the reference forms it, so a body at rest is free of force exactly.
+//     l = l^2 L g after one correction (the residual l^2 - l*l, exact in an fma, times 1 / 2 l;
+//     pd_bond64.cuh). l^2 is formed as the reference forms it, so a body at rest is free of force exactly.
 //   - The failure decision is the reference's eps = (l - L) / L > eps_c. A product decides where
 //     l - L is below eps_c L by more than the rounding of either side; only the bonds beyond
 //     take the division.

@@ -52,6 +52,7 @@ EXPORTS = (
     "pd_mpnn_adam",
     "pd_osb_force_static", "pd_static_last_error",
     "pd_group_create", "pd_group_run_vv", "pd_group_destroy", "pd_tile_info",
+    "pd_eval64",
 )
 
 
@@ -191,6 +192,7 @@ def lib():
         "pd_group_run_vv": [vp, i64, i64, dbl, i32, vp],
         "pd_group_destroy": [vp],
         "pd_tile_info": [vp, vp, vp, vp],
+        "pd_eval64": [i32, i64, vp, vp, vp, i32],
     }
     for name, args in sig.items():
         f = getattr(L, name)
