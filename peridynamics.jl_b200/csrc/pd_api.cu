@@ -85,7 +85,7 @@ static DevParam make_param(const pd_point_params& p, double cs) {
   q.zwaf = (float)q.zwa;
   q.inv_delta = (float)(1.0 / p.delta);
   q.vscale = (float)(1.0 / (p.delta * p.delta * p.delta));
-  q.wratio = (double)q.deltaf / p.delta;
+  q.kap = p.G != 0 ? (3.0 * p.K - 5.0 * p.G) / (15.0 * p.G) : 0.0;
   return q;
 }
 
@@ -290,6 +290,8 @@ static pd_status finish_create(pd_handle* h, int* dnbr_csr, const double* dL, co
     } else {
       PD_TRY(dalloc(h, &h->d.cc32, n));
       PD_TRY(dalloc(h, &h->d.cm32, n));
+      PD_TRY(dalloc(h, &h->d.mlo32, n));
+      PD_CUDA(cudaMemsetAsync(h->d.mlo32, 0, sizeof(float) * n, h->stream));
       PD_CUDA(cudaMemsetAsync(h->d.cc32, 0, sizeof(float2) * n, h->stream));
       PD_CUDA(cudaMemsetAsync(h->d.cm32, 0, sizeof(float2) * n, h->stream));
     }

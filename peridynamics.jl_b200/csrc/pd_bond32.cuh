@@ -101,11 +101,32 @@ __device__ __forceinline__ float dil_term(const Influence& om, const BondP& B, f
   else return om.at<LIN>(B.L, rL) * V * B.L * B.e;
 }
 
-// omega V xi^2, the weighted volume's term
+// What all bonds of a point share moves all of its forces the same way, and on a lattice those of all
+// points: the weighted volume and c1 are therefore not left at their FP32 roundings, nor at those of xi,
+// whose components on a lattice are all off alike (4.7e-8 at a spacing of 1e-3). Velocity error against 64 bits
+// after 60 steps of 975-point coupons at horizons of 2.015, 3.015 and 4.015 spacings: 8.0e-7, 6.2e-7 and 1.3e-6
+// with FP32 sums of omega V xi^2, 4.0e-7, 6.1e-7 and 4.8e-7 so.
+//
+// omega V L^2 in double, the weighted volume's term; LIN: without the factor delta
 template <bool LIN>
-__device__ __forceinline__ float vol_term(const Influence& om, const float4& g, float rL, float V) {
-  const float2 g2 = mul2(xy(g), xy(g));
-  return om.at<LIN>(fabsf(g.w), rL) * V * fmaf(g.z, g.z, g2.x + g2.y);
+__device__ __forceinline__ double vol_term(const Influence& om, float w, float V) {
+  const float L = fabsf(w);
+  if constexpr (LIN) return (double)V * (double)L;
+  else return (double)(om.at<LIN>(L, 0.f) * V) * ((double)L * (double)L);
+}
+
+// a point's weighted volume from the sum of its terms; as stored, in two FP32 parts; and as stored less the
+// terms of bonds that break
+template <bool LIN>
+__device__ __forceinline__ double vol_point(const DevParam& P, double sum) {
+  return LIN ? P.delta * sum : sum;
+}
+__device__ __forceinline__ double vol_stored(const DevBody& d, long long i) {
+  return (double)d.cm32[i].x + (double)d.mlo32[i];
+}
+template <bool LIN>
+__device__ __forceinline__ double vol_less(const DevBody& d, const DevParam& P, long long i, float lost) {
+  return vol_stored(d, i) - vol_point<LIN>(P, (double)lost);
 }
 
 // OSB: omega ((c2_i + c2_j) L + (c1_i + c1_j) e) V / l; LIN: without the factor delta
@@ -116,17 +137,25 @@ __device__ __forceinline__ float osb_pair(const Influence& om, const BondP& B, f
   return f * (V * B.rl);
 }
 
-// OSB: {c1, c2} and the dilatation of a point from its weighted volume w and the sum t of the
-// dilatation's terms. In double: a factor rounded here moves all of the point's bonds the same way
-// (relative error of the forces against 64 bits, 975-point coupon: 9.2e-8 in float, 8.0e-8 so).
+// OSB: {c1, c2} of a point from its weighted volume m and the sum t of the dilatation's terms, with m and
+// the dilatation stored. c2 is formed with the rounded c1: the quotient c1_factor then belongs to both.
 template <bool LIN>
-__device__ __forceinline__ float2 osb_point(const DevParam& P, float w, double t, float& dil) {
-  dil = 0.f;
-  if (w == 0.f) return make_float2(0.f, 0.f);
-  const double rw = (LIN ? P.wratio : 1.0) / (double)w;
-  const double th = 3.0 * rw * (LIN ? P.delta * t : t);
-  dil = (float)th;
-  return make_float2((float)(15.0 * P.G * rw), (float)(th * (3.0 * P.K - 5.0 * P.G) * rw));
+__device__ __forceinline__ void osb_point(const DevBody& d, const DevParam& P, long long i, double m, double t) {
+  float c1 = 0.f, c2 = 0.f, th = 0.f;
+  if (m != 0.0) {
+    const double rm = 1.0 / m, dil = 3.0 * rm * (LIN ? P.delta * t : t);
+    c1 = (float)(15.0 * P.G * rm);
+    c2 = (float)(P.G != 0.0 ? dil * P.kap * (double)c1 : dil * 3.0 * P.K * rm);
+    th = (float)dil;
+  }
+  const float w = (float)m;
+  d.cc32[i] = make_float2(c1, c2);
+  d.cm32[i] = make_float2(w, th);
+  d.mlo32[i] = (float)(m - (double)w);
+}
+// c1 by its rounded value
+__device__ __forceinline__ double c1_factor(const DevBody& d, const DevParam& P, long long i, float c1) {
+  return c1 != 0.f ? 15.0 * P.G / (vol_stored(d, i) * (double)c1) : 1.0;
 }
 
 // the force on a point: its sum times the factor f that all bonds share (in double, as above). A point

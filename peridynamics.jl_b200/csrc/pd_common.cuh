@@ -68,10 +68,7 @@ struct DevParam {
   float deltaf, bcf, epscf, Gf, Kf, lambdaf, muf, betaf, zwaf;
   float inv_delta;  // 1 / delta (FP32 correspondence scaling)
   float vscale;     // 1 / delta^3 (FP32 correspondence scaling)
-  // (float)delta / delta: the packed FP32 OSB kernels take the linear influence function's factor delta
-  // out of the sums of forces and dilatations and apply it in double, but sum the weighted volume with
-  // (float)delta; the quotient belongs to the inverse weighted volume, else it moves all forces of a body
-  double wratio;
+  double kap;       // (3 K - 5 G) / (15 G): c2 = theta kap c1 of OSB (0 where G is 0)
 };
 
 struct Ctrl {
@@ -121,6 +118,7 @@ struct DevBody {
   double4* coef64;   // OSB FP64: {c1, c2, wvol, dil}
   float2* cc32;      // OSB FP32: {c1, c2}
   float2* cm32;      // OSB FP32: {wvol, dil}
+  float* mlo32;      // OSB FP32, packed kernels: what wvol lacks of the weighted volume
   float4* uhi;       // FP32 path: {(float)u, V}
   float4* ulo;       // FP32 path: {(float)(u - hi), 0}
   double* F64;       // CMat FP64: deformation gradient F (9 per point, column-major)

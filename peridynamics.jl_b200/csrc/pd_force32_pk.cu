@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256, PD_MINB_QB) k_osb_b32q(DevBody d, int kst
       }
     }
     if (valid) {
-      store_force(d, i, kstep, LIN ? P.delta : 1.0, txy, tz);
+      store_force(d, i, kstep, (LIN ? P.delta : 1.0) * c1_factor(d, P, i, ci.x), txy, tz);
     }
   }
 }
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256, PD_MINB_QA) k_osb_a32q(DevBody d, int kst
     const int* pn = d.nbr + sbase + lane;
     const float4* pg = d.geo + sbase + lane;
     unsigned* pw = d.bits + (sbase >> 5);
-    KSum2 mt, tmt;  // the sums of the segment and of the point
+    double sm = 0.0, tm = 0.0;  // the sums of the segment and of the point
     KSum1 th, tth;
     float dm = 0.f, tdm = 0.f;
     int na = 0;
@@ -183,13 +183,9 @@ __global__ void __launch_bounds__(256, PD_MINB_QA) k_osb_a32q(DevBody d, int kst
         bond_pk(g, hj, u ? lj1 : lj0, own, B);
         const float rL = bond_rl(g.w);
         const bool act = stays(a, B.e * rL, epsc, g.w);
-        const float th_b = act ? dil_term<LIN>(om, B, rL, hj.w) : 0.f;
-        if (FULLM) {
-          mt.add(make_float2(act ? vol_term<LIN>(om, g, rL, hj.w) : 0.f, th_b));
-        } else {
-          th.add(th_b);
-          if (a && !act) dm += vol_term<LIN>(om, g, rL, hj.w);
-        }
+        th.add(act ? dil_term<LIN>(om, B, rL, hj.w) : 0.f);
+        if (FULLM) sm += act ? vol_term<LIN>(om, g.w, hj.w) : 0.0;
+        else if (a && !act) dm += (float)vol_term<LIN>(om, g.w, hj.w);
         if (u) act1 = act; else act0 = act;
       }
       na += (int)act0 + (int)act1;
@@ -200,28 +196,19 @@ __global__ void __launch_bounds__(256, PD_MINB_QA) k_osb_a32q(DevBody d, int kst
         if (two && c1 != w1) pw[r + 1] = c1;
       }
       if ((r + 2) % SEG32 == 0 || r + 2 >= rows) {
-        join(tmt, mt);
+        tm += sm;
         join(tth, th);
         tdm += dm;
-        mt = KSum2();
+        sm = 0.0;
         th = KSum1();
         dm = 0.f;
       }
     }
     if (valid) {
-      float wv;
-      double tv;
-      if (FULLM) {
-        wv = tmt.value().x;
-        tv = (double)tmt.s.y + (double)tmt.n.y;
-      } else {
-        const float m0 = d.cm32[i].x;
-        wv = tdm != 0.f ? m0 - tdm : m0;
-        tv = (double)tth.s + (double)tth.n;
-      }
-      float dil;
-      d.cc32[i] = osb_point<LIN>(P, wv, tv, dil);
-      d.cm32[i] = make_float2(wv, dil);
+      double m;
+      if (FULLM) m = vol_point<LIN>(P, tm);
+      else m = tdm != 0.f ? vol_less<LIN>(d, P, i, tdm) : vol_stored(d, i);
+      osb_point<LIN>(d, P, i, m, (double)tth.s + (double)tth.n);
       d.n_active[i] = na;
     }
   }

@@ -298,8 +298,8 @@ struct ForceSum {
   }
 };
 
-// the sums of OSB phase A: dilatation; in full also the weighted volume (packed with it), else what
-// the stored one loses; the active bonds in full, else those that break
+// the sums of OSB phase A: dilatation; in full also the weighted volume (in double), else what the stored
+// one loses; the active bonds in full, else those that break
 template <bool FULLM>
 struct DilSum {
   KSum1 th;
@@ -313,10 +313,12 @@ struct DilSum {
 };
 template <>
 struct DilSum<true> {
-  KSum2 mt;
+  double m = 0.0;
+  KSum1 th;
   int na = 0;
   __device__ __forceinline__ void join(const DilSum& o) {
-    pack::join(mt, o.mt);
+    m += o.m;
+    pack::join(th, o.th);
     na += o.na;
   }
 };
@@ -385,12 +387,10 @@ __global__ void __launch_bounds__(256, MT_A) k_osb_a32s(DevBody d, int kstep) {
       bond_pk(p.g[u], hj, t.lo(p.key[u]), own, B);
       const float rL = st.rL(p, u);
       act[u] = stays(p.a[u], B.e * rL, epsc, p.g[u].w);
-      const float th_b = act[u] ? dil_term<LIN>(om, B, rL, hj.w) : 0.f;
+      s.th.add(act[u] ? dil_term<LIN>(om, B, rL, hj.w) : 0.f);
       if constexpr (FULLM) {
-        s.mt.add(make_float2(act[u] ? vol_term<LIN>(om, p.g[u], rL, hj.w) : 0.f, th_b));
+        s.m += act[u] ? vol_term<LIN>(om, p.g[u].w, hj.w) : 0.0;
         s.na += (int)act[u];
-      } else {
-        s.th.add(th_b);
       }
     }
     const unsigned c0 = __ballot_sync(0xffffffffu, act[0]), c1 = __ballot_sync(0xffffffffu, act[1]);
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(256, MT_A) k_osb_a32s(DevBody d, int kstep) {
 #pragma unroll
         for (int u = 0; u < 2; u++)
           if (p.a[u] && !act[u]) {
-            s.dm += vol_term<LIN>(om, p.g[u], st.rL(p, u), t.hi(p.key[u]).w);
+            s.dm += (float)vol_term<LIN>(om, p.g[u].w, t.hi(p.key[u]).w);
             s.na++;
           }
       }
@@ -407,19 +407,10 @@ __global__ void __launch_bounds__(256, MT_A) k_osb_a32s(DevBody d, int kstep) {
     }
   });
   if (t.valid && t.part == 0) {
-    float wv;
-    double tv;
-    if constexpr (FULLM) {
-      wv = S.mt.value().x;
-      tv = (double)S.mt.s.y + (double)S.mt.n.y;
-    } else {
-      const float m0 = d.cm32[t.i].x;
-      wv = S.dm != 0.f ? m0 - S.dm : m0;
-      tv = (double)S.th.s + (double)S.th.n;
-    }
-    float dil;
-    d.cc32[t.i] = osb_point<LIN>(P, wv, tv, dil);
-    d.cm32[t.i] = make_float2(wv, dil);
+    double m;
+    if constexpr (FULLM) m = vol_point<LIN>(P, S.m);
+    else m = S.dm != 0.f ? vol_less<LIN>(d, P, t.i, S.dm) : vol_stored(d, t.i);
+    osb_point<LIN>(d, P, t.i, m, (double)S.th.s + (double)S.th.n);
     if (FULLM) d.n_active[t.i] = S.na;
     else if (S.na) d.n_active[t.i] -= S.na;
   }
@@ -446,7 +437,7 @@ __global__ void __launch_bounds__(256, MT_B) k_osb_b32s(DevBody d, int kstep) {
     }
   });
   if (t.valid && t.part == 0)
-    store_force(d, t.i, kstep, LIN ? P.delta : 1.0, S.xy, S.z);
+    store_force(d, t.i, kstep, (LIN ? P.delta : 1.0) * c1_factor(d, P, t.i, ci.x), S.xy, S.z);
 }
 
 // the sums of correspondence phase A and its count; not cut into segments (their sums would take
