@@ -30,3 +30,22 @@ def test_autotune_times_a_kernel_once(name):
     dev.force()
     assert np.abs(dev.field("b_int").T - ob.b_int).max() < 2e-5 * np.abs(ob.b_int).max()
     dev.close()
+
+
+def test_tuning_leaves_nothing_of_other_kernels_behind():
+    """The kernels timed on the way store weighted volumes with their own roundings; the chosen ones sum
+    theirs anew."""
+    body = box(MATERIALS["OSB"](), 40, 30, 20, 3.015, jitter=0.05)
+    u = deform(body._pos)
+    dev, ref = (pd.DeviceBody(body, precision="fp32") for _ in range(2))
+    dev.set_state(displacement=u)
+    dev.autotune()
+    group, block, pipe = dev.mapping()
+    ref.set_mapping(group, block)
+    ref.set_pipeline(pipe)
+    ref.set_state(displacement=u)
+    for d in (dev, ref):
+        d.force()
+    assert np.array_equal(dev.field("b_int"), ref.field("b_int"))
+    dev.close()
+    ref.close()

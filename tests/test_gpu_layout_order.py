@@ -53,8 +53,8 @@ def test_staged_variants_and_back(name, pipe):
             assert np.array_equal(dev.field("bond_active"), ref.field("bond_active"))
             dev.set_pipeline(5)
             assert dev.tile_info() == tiles
-            for d in (dev, ref):   # the staged kernels sum the weighted volumes anew: so do both
-                d.set_state(bond_active=ref.field("bond_active"))
+            # weighted volumes of other kernels are not kept: dev sums its own anew, and so does ref
+            ref.set_state(bond_active=ref.field("bond_active"))
     for f in ("b_int", "bond_active", "n_active_bonds", "displacement"):
         assert np.array_equal(dev.field(f), ref.field(f)), f
     assert 0.0 < dev.field("bond_active").mean() < 1.0
