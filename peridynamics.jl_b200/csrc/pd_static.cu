@@ -124,8 +124,8 @@ __global__ void __launch_bounds__(256) k_static_osb_a(StaticArgs a) {
     s_diff(a.x, xi, j, d);
     s_diff(a.X, Xi, j, D);
     const double l2 = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2];
-    // two points in one place: no reciprocal of the length, but a dilatation
-    const double e = l2 < DBL_MIN ? -L : sqrt_of(l2, rsqrt3(l2)) - L;
+    // DBL_MIN: two points in one place have no reciprocal of the length, but a dilatation
+    const double e = sqrt_of(l2, rsqrt3(l2 + DBL_MIN)) - L;
     if (!(L > 0 && e < thr * L) && (sqrt(l2) - L) / L > a.epsc && a.fail_permit[b]) {
       a.bond_active[b] = 0;
       act = 0;
