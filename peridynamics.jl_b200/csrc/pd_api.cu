@@ -90,7 +90,6 @@ static DevParam make_param(const pd_point_params& p, double cs) {
   q.zwaf = (float)q.zwa;
   q.inv_delta = (float)(1.0 / p.delta);
   q.vscale = (float)(1.0 / (p.delta * p.delta * p.delta));
-  q.kap = p.G != 0 ? (3.0 * p.K - 5.0 * p.G) / (15.0 * p.G) : 0.0;
   return q;
 }
 

@@ -105,7 +105,7 @@ __device__ __forceinline__ float dil_term(const Influence& om, const BondP& B, f
 // points: the weighted volume and c1 are therefore not left at their FP32 roundings, nor at those of xi,
 // whose components on a lattice are all off alike (4.7e-8 at a spacing of 1e-3). Velocity error against 64 bits
 // after 60 steps of 975-point coupons at horizons of 2.015, 3.015 and 4.015 spacings: 8.0e-7, 6.2e-7 and 1.3e-6
-// with FP32 sums of omega V xi^2, 4.0e-7, 6.1e-7 and 4.8e-7 so.
+// with FP32 sums of omega V xi^2, 4.3e-7, 5.3e-7 and 4.7e-7 so.
 //
 // omega V L^2 in double, the weighted volume's term; LIN: without the factor delta
 template <bool LIN>
@@ -137,25 +137,40 @@ __device__ __forceinline__ float osb_pair(const Influence& om, const BondP& B, f
   return f * (V * B.rl);
 }
 
+// v in FP32, up or down by a draw that the reference position decides: a value that many points share is
+// rounded to either side in the proportion that keeps its mean. (To nearest, c1 of a lattice's inner points moved
+// all of their forces by up to 6e-8. Any factor of a point's own on its force sum would keep two points' forces
+// on each other from being opposite.) The draw: the position's bits through the mixing steps of splitmix64
+__device__ __forceinline__ float round_drawn(double v, const double4& X) {
+  const float lo = __double2float_rd(v), hi = __double2float_ru(v);
+  unsigned long long h = 0x9E3779B97F4A7C15ull;
+  const double x[3] = {X.x, X.y, X.z};
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    h ^= (unsigned long long)__double_as_longlong(x[k]);
+    h = (h ^ (h >> 30)) * 0xBF58476D1CE4E5B9ull;
+    h = (h ^ (h >> 27)) * 0x94D049BB133111EBull;
+    h ^= h >> 31;
+  }
+  const double u = (double)(unsigned)(h >> 32) * 0x1p-32;
+  return v - (double)lo > u * ((double)hi - (double)lo) ? hi : lo;
+}
+
 // OSB: {c1, c2} of a point from its weighted volume m and the sum t of the dilatation's terms, with m and
-// the dilatation stored. c2 is formed with the rounded c1: the quotient c1_factor then belongs to both.
+// the dilatation stored
 template <bool LIN>
 __device__ __forceinline__ void osb_point(const DevBody& d, const DevParam& P, long long i, double m, double t) {
   float c1 = 0.f, c2 = 0.f, th = 0.f;
   if (m != 0.0) {
     const double rm = 1.0 / m, dil = 3.0 * rm * (LIN ? P.delta * t : t);
-    c1 = (float)(15.0 * P.G * rm);
-    c2 = (float)(P.G != 0.0 ? dil * P.kap * (double)c1 : dil * 3.0 * P.K * rm);
+    c1 = round_drawn(15.0 * P.G * rm, d.X0[i]);
+    c2 = (float)(dil * (3.0 * P.K - 5.0 * P.G) * rm);
     th = (float)dil;
   }
   const float w = (float)m;
   d.cc32[i] = make_float2(c1, c2);
   d.cm32[i] = make_float2(w, th);
   d.mlo32[i] = (float)(m - (double)w);
-}
-// c1 by its rounded value
-__device__ __forceinline__ double c1_factor(const DevBody& d, const DevParam& P, long long i, float c1) {
-  return c1 != 0.f ? 15.0 * P.G / (vol_stored(d, i) * (double)c1) : 1.0;
 }
 
 // the force on a point: its sum times the factor f that all bonds share (in double, as above). A point

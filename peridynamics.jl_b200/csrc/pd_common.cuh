@@ -68,7 +68,6 @@ struct DevParam {
   float deltaf, bcf, epscf, Gf, Kf, lambdaf, muf, betaf, zwaf;
   float inv_delta;  // 1 / delta (FP32 correspondence scaling)
   float vscale;     // 1 / delta^3 (FP32 correspondence scaling)
-  double kap;       // (3 K - 5 G) / (15 G): c2 = theta kap c1 of OSB (0 where G is 0)
 };
 
 struct Ctrl {

@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256, PD_MINB_QB) k_osb_b32q(DevBody d, int kst
       }
     }
     if (valid) {
-      store_force(d, i, kstep, (LIN ? P.delta : 1.0) * c1_factor(d, P, i, ci.x), txy, tz);
+      store_force(d, i, kstep, LIN ? P.delta : 1.0, txy, tz);
     }
   }
 }

@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(256, MT_B) k_osb_b32s(DevBody d, int kstep) {
     }
   });
   if (t.valid && t.part == 0)
-    store_force(d, t.i, kstep, (LIN ? P.delta : 1.0) * c1_factor(d, P, t.i, ci.x), S.xy, S.z);
+    store_force(d, t.i, kstep, LIN ? P.delta : 1.0, S.xy, S.z);
 }
 
 // the sums of correspondence phase A and its count; not cut into segments (their sums would take
