@@ -543,9 +543,12 @@ pd_status pd_mpnn_adam(pd_mpnn *net, float lr);
  * volume [n], bond_offsets [n+1], neighbors, bond_length, fail_permit [n_bonds];
  * bond_active [n_bonds] is updated by the failure test; b_int [3n] and n_active [n] are
  * written. Bond states need not agree in the two directions of a pair: the term of
- * neighbour j on point i uses j's own bond j -> i (its state and length), found by a binary
- * search of j's sorted list, as the reference's scatter does; a neighbour without a bond to
- * i adds nothing. Kernels run on `stream` (NULL: the default stream); the call does not
+ * neighbour j on point i uses j's own bond j -> i (its state and length), found in j's sorted
+ * list at the mirrored place or else by a binary search, as the reference's scatter does; a
+ * neighbour without a bond to i adds nothing. The arithmetic is that of the FP64 mappings off
+ * the serial order: 8, 16 or 32 lanes share a point, by n, and their sums are added in a fixed
+ * tree, so that results do not depend on the schedule but differ from the serial order's
+ * in the last bits. Kernels run on `stream` (NULL: the default stream); the call does not
  * wait. A CUDA error left pending by earlier work of the calling thread is reported
  * (PD_ERR_CUDA) before anything is launched and stays pending.
  * Limit: n <= 262144 points. The per-point coefficients live in a static device array of

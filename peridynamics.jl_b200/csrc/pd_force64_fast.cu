@@ -1,4 +1,7 @@
-// pd_force64_fast.cu -- FP64 force kernels of every mapping but the serial order.
+// pd_force64_fast.cu -- FP64 force kernels off the serial order that gather from global memory:
+// correspondence, lane groups, several parameter sets, EnergySurfaceCorrection, OSB phase B of bodies small
+// enough to split their slices, and BB and OSB bodies without tiles. Others run pd_tile64.cu, with the same
+// arithmetic and order of the sums: the same bits.
 //
 // What bounds them: per bond 12 bytes of stream (neighbour index and reference length), 32 to
 // 144 bytes gathered through L1 from the neighbour's point records, and the FP64 pipe (two warp
@@ -24,7 +27,7 @@
 //     with eta - F xi = du - H xi. A and beta are kept in five planes of double2 (structure of
 //     arrays), so that the 32 lanes of a warp read consecutive 16-byte words.
 //
-// Time a step, lattices at a horizon of 3.015 spacings, before and after (one lane per point, us,
+// Time a step, lattices at a horizon of 3.015 spacings, before and after (one lane per point, without tiles, us,
 // CUDA graphs): 3,200 points BB 55.6 -> 10.9, OSB 129 -> 17.5, CMat 237 -> 24; 27,347 points BB 70
 // -> 23, OSB 163 -> 42, CMat 301 -> 77; 125,000 points BB 153 -> 101, OSB 401 -> 190, CMat 920 ->
 // 281; 397,243 points BB 376 -> 268, OSB 1049 -> 498.

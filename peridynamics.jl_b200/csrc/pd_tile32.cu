@@ -16,9 +16,9 @@
 // are those of pd_force32_pk.cu: the same bits.
 //
 // Time of a step, lattices at a horizon of 3.015 spacings, packed kernels before and tiles (us, CUDA
-// graphs): OSB 1M points 1003 -> 633, 4.24M 4381 -> 2600, jittered 1M 1056 -> 955; BB 1M 501 -> 356;
-// CMat 320k 464 -> 314, 125k 232 -> 184. Against the one-row kernels of an untuned body: OSB 975 points
-// 65 -> 15, 27,347 105 -> 37, 64,000 185 -> 69; CMat 64,000 212 -> 87. OSB phase A issues 75 % of its
+// graphs): OSB 1M points 1003 -> 635, 4.24M 4381 -> 2694, jittered 1M 1056 -> 949; BB 1M 501 -> 362;
+// CMat (variant 5) 320k 464 -> 317, 125k 232 -> 185. Against the one-row kernels of an untuned body: OSB 975
+// points 65 -> 17, 27,347 105 -> 38, 64,000 185 -> 66; CMat 64,000 212 -> 88. OSB phase A issues 75 % of its
 // slots with the L1 pipe at 63 %: arithmetic and the neighbour and class records read from shared
 // memory (12 wavefronts a row) are what is left. With the full geometry stream DRAM is at 56 %, and
 // copying it ahead asynchronously (4 to 8 rows in shared memory) changed no time by more than 3 %.
@@ -323,8 +323,8 @@ struct DilSum<true> {
   }
 };
 
-// Resident blocks of 256 threads per SM, measured on 1M-point blocks (us a launch): BB 4 blocks (64
-// registers) 295 / 3 361 / 5 426; OSB phase A 4 blocks 287 / 3 360 / 5 406, full geometry stream 438 /
+// Resident blocks of 256 threads per SM, measured on 1M-point blocks with the first form of these kernels
+// (us a launch): BB 4 blocks (64 registers) 295 / 3 361 / 5 426; OSB phase A 4 blocks 287 / 3 360 / 5 406, full geometry stream 438 /
 // 476 / 701; OSB phase B 3 blocks (80 registers) 336 / 4 377; CMat phase A 3 blocks 403 / 2 507, with
 // compensated sums 2 blocks 525, phase B 2 blocks (tiles of 72 bytes a point fill the SM) 537 / 3 579.
 constexpr int MT_BB = 4, MT_A = 4, MT_B = 3, MT_CA = 3, MT_CAK = 2, MT_CB = 2;
