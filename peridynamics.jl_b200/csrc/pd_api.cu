@@ -165,8 +165,8 @@ static bool wants_places(const pd_handle* h) {
 }
 
 // Bodies with one lane per point gather from tiles in shared memory (FP64: BB and OSB) and, in FP32
-// on a regular lattice, read a bond's geometry as one byte. Both are made once per layout; a body without tiles or
-// classes, or without the memory for them, runs the kernels that its bond-stream variant names.
+// on a regular lattice, read a bond's geometry as one byte. Both are made once per layout; a body without tiles,
+// or without the memory for them, gathers from global memory, one without classes reads 16 bytes.
 static pd_status ensure_tiles(pd_handle* h) {
   if (h->tiles_tried || h->d.lg != 1 || h->d.pt == nullptr || h->multi)
     return PD_OK;
@@ -333,11 +333,8 @@ static pd_status finish_create(pd_handle* h, int* dnbr_csr, const double* dL, co
   return PD_OK;
 }
 
-// moves every bond array into the layout with G lanes per point, one lane in the order that the handle's
-// kernels want
-static pd_status relayout(pd_handle* h, int G) {
-  const bool places = G == 1 && wants_places(h) && h->pt != nullptr;
-  if (G == h->d.lg && places == (h->d.pt != nullptr)) return PD_OK;
+// every bond array in the layout with G lanes per point, places: in the order of the tiles
+static pd_status move_bonds(pd_handle* h, int G, bool places) {
   PD_CUDA(cudaStreamSynchronize(h->stream));
   DevBody a = h->d, b = h->d;
   long long* soff = nullptr;
@@ -415,6 +412,25 @@ static pd_status relayout(pd_handle* h, int G) {
   h->tiles_tried = false;
   h->d = b;
   h->nslots = nslots;
+  return PD_OK;
+}
+
+// the layout with G lanes per point, one lane in the order that the handle's kernels want. On failure, for want
+// of memory among others, the body keeps its layout and what was allocated for the other is given back
+static pd_status relayout(pd_handle* h, int G) {
+  const bool places = G == 1 && wants_places(h) && h->pt != nullptr;
+  if (G == h->d.lg && places == (h->d.pt != nullptr)) return PD_OK;
+  const size_t kept = h->allocs.size();
+  const pd_status st = move_bonds(h, G, places);
+  if (st != PD_OK) {
+    cudaStreamSynchronize(h->stream);
+    while (h->allocs.size() > kept) {
+      cudaFree(h->allocs.back());
+      h->allocs.pop_back();
+    }
+    cudaGetLastError();  // the caller has st; the next check of a launch is not to find it
+    return st;
+  }
   drop_graphs(h);
   return ensure_tiles(h);
 }
@@ -1171,6 +1187,7 @@ static pd_status run_block_graph(pd_handle* h, int steps, double dto) {
     cudaGraph_t graph;
     long long before = h->launches;
     PD_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+    cudaGetLastError();  // of earlier calls
     issue_steps(h, steps, dto, nullptr);
     const cudaError_t le = cudaGetLastError();  // a launch that was refused
     cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
@@ -1361,6 +1378,7 @@ extern "C" pd_status pd_group_run_vv(pd_group* g, int64_t first_step, int64_t n_
         cudaGraph_t graph;
         cudaError_t e = cudaStreamBeginCapture(origin, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
+          cudaGetLastError();  // of earlier calls
           group_issue(g, steps, dto);
           const cudaError_t le = cudaGetLastError();  // a launch that was refused
           e = cudaStreamEndCapture(origin, &graph);
@@ -1541,17 +1559,17 @@ extern "C" pd_status pd_autotune(pd_handle* h, int32_t* group_out, int32_t* bloc
   const bool f32 = h->precision == PD_PREC_FP32_KAHAN, corr = h->material == PD_MAT_CMAT;
   for (int G : {1, 4, 32}) {
     // the variants to time: plain loads, then (FP32 BB / OSB) the two-row kernels, then (one lane per point)
-    // the TMA-staged bond stream and the packed kernels
+    // the packed kernels and the TMA-staged bond stream, which wants another order of the points
     std::vector<int> pipes{0};
     if (f32 && !corr) pipes.push_back(4);
     if (f32 && G == 1) {
-      if (!corr) pipes.insert(pipes.end(), {1, 2, 3});
       pipes.push_back(5);
+      if (!corr) pipes.insert(pipes.end(), {1, 2, 3});
     }
     for (int pipe : pipes) {
       h->cfg.group = G; h->cfg.exact = false; h->cfg.pipe = pipe;
       pd_status st = relayout(h, G);
-      if (st == PD_ERR_OOM) { cudaGetLastError(); break; }  // no room for a second layout
+      if (st == PD_ERR_OOM) break;  // no room for a second layout
       if (st != PD_OK) return give_up(st);
       const bool tma = pipe >= 1 && pipe <= 3;
       if (tma && !tma_supported(h->d)) continue;
@@ -1580,7 +1598,7 @@ extern "C" pd_status pd_autotune(pd_handle* h, int32_t* group_out, int32_t* bloc
   for (int round = 0; round < 2 && cands.size() > 1; round++)
     for (auto& c : cands) {
       h->cfg = c.c;
-      if (relayout(h, c.c.group) != PD_OK) { cudaGetLastError(); continue; }
+      if (relayout(h, c.c.group) != PD_OK) continue;
       float ms;
       pd_status ts = time_cfg(&ms);
       if (ts != PD_OK) return give_up(ts);
@@ -1722,16 +1740,14 @@ extern "C" pd_status pd_set_pipeline(pd_handle* h, int32_t pipe) {
   sum_anew(h);
   drop_graphs(h);
   const pd_status st = relayout(h, h->d.lg);
-  if (st == PD_ERR_OOM) { cudaGetLastError(); return PD_OK; }  // any order will do
-  return st;
+  return st == PD_ERR_OOM ? PD_OK : st;  // any order will do
 }
 
 // pd_esc_init: the bond factors have no place in the tiles
 pd_status pd_without_tiles(pd_handle* h) {
   h->esc = true;
   const pd_status st = relayout(h, h->d.lg);
-  if (st == PD_ERR_OOM) { cudaGetLastError(); return PD_OK; }
-  return st;
+  return st == PD_ERR_OOM ? PD_OK : st;
 }
 
 // helpers shared with pd_nk.cu
