@@ -1736,6 +1736,7 @@ extern "C" pd_status pd_set_pipeline(pd_handle* h, int32_t pipe) {
     return fail(PD_ERR_ARG, "the packed-pair kernels are FP32 ones");
   if (pipe >= 1 && pipe <= 3 && (h->precision != PD_PREC_FP32_KAHAN || !tma_supported(h->d)))
     return fail(PD_ERR_ARG, "the staged bond stream needs the FP32 path, one lane per point and BB or OSB");
+  PD_CUDA(cudaSetDevice(h->device));
   h->cfg.pipe = pipe;
   sum_anew(h);
   drop_graphs(h);
