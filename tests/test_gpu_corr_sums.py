@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("jitter", [0.0, 0.05])
-@pytest.mark.parametrize("m", [5.015, 5.6])   # the second phase of 5.6 spacings does not fit a tile
+@pytest.mark.parametrize("m", [5.015, 5.6])   # tiles of 1,906 and 2,081 points: both phases fit
 def test_gradient_of_a_uniform_deformation(jitter, m):
     body = box(pd.CMaterial(), 17, 16, 15, m, jitter)
     G = np.array([[3.1e-3, 1.3e-3, -0.7e-3], [0.9e-3, -2.3e-3, 1.9e-3], [1.1e-3, 0.3e-3, 2.7e-3]])
